@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -12,6 +13,7 @@
 #include "../../include/flups.h"
 #include "fast_dft.h"
 #include "green.cuh"
+#include "mix_dft.h"
 #include "pass_desc.h"
 
 #define FLB_CHECK(cond, ...)                                                        \
@@ -216,8 +218,19 @@ struct Solver {
     const void* twiddle_plain(int L, bool f64);   // W_L^q, q < L
     // later-stage twiddles of an n-point register DFT with first radix r1 (0: the default of the precision)
     const void* stage_table(int n, bool f64, int r1 = 0);
-    // 0 none, 1 column c2c, 2 row r2c/c2r, 3 column r2c/c2r, 4 row r2r, 5 fused row
+    // 0 general line pass, 1 column c2c, 2 row r2c/c2r, 3 column r2c/c2r, 4 row r2r, 5 fused row, 6 mixed radix
     int fast_kind(const flb::PassArgs& A, bool f64, bool in_f64, bool out_f64) const;
+    int reg_kind(const flb::PassArgs& A, bool f64, bool in_f64, bool out_f64) const;
+    // mixed-radix passes: the operation (MixOp) that can run a pass, or -1; its launch arguments and twiddles
+    int mix_op(const flb::PassArgs& A, bool f64, bool in_f64, bool out_f64) const;
+    void mix_args(const flb::PassArgs& A, int op, bool f64, bool in_f64, bool out_f64, flb::MixArgs& m) const;
+    const void* mix_table(const flb::MixPlan& p, bool f64);
+    const void* type4_table(int N, bool f64);
+    void* upload_table(const std::vector<double>& w, bool f64);
+    const flb::MixPlan* mix_plan_of(int M, int op, bool f64) const;
+    mutable std::map<std::array<int, 3>, flb::MixPlan> mix_plans;         // per length, operation and precision
+    mutable std::map<std::array<int, 7>, std::array<int, 2>> mix_tiles;   // and per extents: lines, threads per line
+    bool use_mix = true;                  // false while the no-allocation solve plans its passes
     // arguments of a fast launch, all but the twiddle tables; mode of a column pass
     void fast_args(const flb::PassArgs& A, int kind, bool in_f64, bool out_f64, flb::ColArgs& c, flb::RowArgs& r, int& mode) const;
     void launch_fast(const flb::PassArgs& A, int kind, bool f64, bool in_f64, bool out_f64);

@@ -1,0 +1,99 @@
+// Mixed-radix line passes for the transform lengths the register DFTs do not
+// take: arguments, factorisation and launcher (kernels in mix_dft_impl.cuh).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace flb {
+
+// What one pass does with its lines.  "Pairs" carry two real lines a, b in one
+// complex transform z = a + i b and part them at the frequency side.
+enum MixOp : int {
+    MX_C2C_F = 0,  // forward complex DFT
+    MX_C2C_I = 1,  // inverse complex DFT
+    MX_R2C = 2,    // pairs of real lines -> half spectra
+    MX_C2R = 3,    // half spectra -> pairs of real lines
+    MX_FUSED = 4,  // forward complex DFT, Green's multiply, inverse DFT, in place
+    // r2r kinds (FFTW size N); pairs but for type 4
+    MX_T2 = 5,     // DCT-II / DST-II, M = N
+    MX_T3 = 6,     // DCT-III / DST-III, M = N
+    MX_T1 = 7,     // DCT-I (M = 2 (N - 1)) / DST-I (M = 2 (N + 1))
+    MX_T4 = 8,     // DCT-IV / DST-IV of even N, M = N / 2
+    // a real last direction: transform, Green's multiply, inverse transform, in place
+    MX_FUSED_R = 9,    // r2c, c2r
+    MX_FUSED_23 = 10,  // type II, type III
+    MX_FUSED_32 = 11,  // type III, type II
+    MX_FUSED_11 = 12,  // type I twice
+    MX_FUSED_44 = 13,  // type IV twice
+    MX_ROT = 14,       // forward complex DFT of three components, curl and Green's multiply, inverse DFT, in place
+};
+// two real lines per complex transform
+constexpr bool mix_pairs(int op) { return op == MX_R2C || op == MX_C2R || (op >= MX_T2 && op <= MX_FUSED_11 && op != MX_T4); }
+// lines of a tile's line position held together
+constexpr int mix_planes(int op) { return op == MX_ROT ? 3 : 1; }
+// the last stage takes the butterflies of k and M - k together
+constexpr bool mix_mirrors(int op) {
+    return op == MX_R2C || op == MX_C2R || op == MX_T2 || op == MX_T3 || op == MX_FUSED_R || op == MX_FUSED_23 || op == MX_FUSED_32;
+}
+
+constexpr int kMixStages = 4;
+constexpr int kMixThreads = 256;
+
+// Stage s of the decimation in frequency: radix R on sub-blocks of R * nn
+// points (nn points are left of each after it); Q = product of the radices
+// before it, so a line has Q * nn butterflies.
+struct MixStage {
+    int R, nn, Q;
+    unsigned qmul;  // ceil(2^32 / Q): x / Q = umulhi(x, qmul) for x Q < 2^32 (Q = 1: not used)
+    int tw;         // first entry of the stage's twiddles W_{R nn}^{k m} at (k - 1) nn + m, 0 < k < R, m < nn
+};
+
+struct MixPlan {
+    int M, ns;              // line length, number of stages
+    int s1;                 // distance in shared memory between the first digit's blocks (odd)
+    int len;                // elements a line takes in shared memory
+    int ntw;                // complex entries of the stage twiddles
+    MixStage st[kMixStages];
+};
+
+struct MixArgs {
+    const void* in;
+    void* out;
+    MixPlan pl;
+    const void* tw;                        // stage twiddles, working precision
+    int na, nb;                            // line positions: a (lanes of the column passes), b
+    int n_src, n_store;                    // source / stored extent of a line
+    int64_t in_sl, in_sa, in_sb, in_sc;    // element strides: along the line, a, b, component
+    int64_t out_sl, out_sa, out_sb, out_sc;
+    int in64, out64;                       // a real side holds doubles
+    int period;                            // output index that receives a copy of output 0, or -1
+    // r2r kinds: pre / post twiddles W_4N^k (type IV: W_8N^{4j+1} in tw8), the place of the source in the padded
+    // line and of the stored part in the output line, and per component: FFTW's size, the odd (DST) kind, first
+    // input and output element of the transform in its line, first spectral element of a fused pass, output
+    // elements (of the stored part) set to zero, or -1
+    const void *tw4, *tw8;
+    int fieldstart, store_off, lda;
+    int N[3], dst[3], fi[3], fo[3], go[3], z0[3], z1[3];
+    int tx, P;                             // tile: lines per CTA (pairs count once), threads per line
+    // Green's multiply
+    const void* green;
+    int64_t g_sa, g_sb, g_sl;
+    int f_a, f_b, f_l;                     // fold lengths (0 = none)
+    // curl symbols K_{d,c}(i) at (3 d + c) kstr + i; the directions of a, b and the line
+    const void* ksym;
+    int kstr, ax_a, ax_b, ax_l;
+};
+
+// Factorisation of M for a pass of operation `op`; false when M has a prime
+// factor above 13, or does not split into two to four of the radices.
+bool mix_plan(int M, int op, int f64, MixPlan& p);
+// W_{R nn}^{k m} of entry e of the stage twiddles: exponent and root order
+void mix_twiddle_exponent(const MixPlan& p, int e, int* q, int* n);
+// lines per CTA and threads per line (a.tx, a.P) for the pass's extents
+void mix_tile(MixArgs& a, int f64, int op, bool rows, int64_t ncomp);
+// rows: lines along the lanes' direction (x); ncomp: grid z
+cudaError_t launch_mix(int f64, int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
+// whether one line position of the pass fits in shared memory
+bool mix_fits(const MixPlan& p, int op, int f64);
+
+}  // namespace flb

@@ -114,6 +114,13 @@ extern "C" int flups_solve_noalloc(Solver* s, double* field, double* rhs, int ty
         }
     }
 
+    // the mixed-radix passes keep their twiddles in tables of their own: this
+    // call runs the general line pass for those lengths
+    struct NoMix {
+        Solver* s;
+        explicit NoMix(Solver* sv) : s(sv) { s->use_mix = false; }
+        ~NoMix() { s->use_mix = true; }
+    } no_mix(s);
     // the passes of one solve, planned on the host with the work arrays placed in the scratch array
     void* keep[2] = {s->buf[0], s->buf[1]};
     s->buf[0] = wb[0];

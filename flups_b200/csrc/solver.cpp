@@ -20,6 +20,7 @@
 
 #include "fast_dft.h"
 #include "host.hpp"
+#include "mix_dft.h"
 #include "rot.h"
 
 using namespace flb;
@@ -222,7 +223,7 @@ void Solver::plan_xlast() {
         do_fft_backward_fused(nullptr, type, 1);
         bool ok = !dry_fast.empty();
         for (size_t i = 0; i < dry_fast.size(); ++i) {
-            if (dry_fast[i] == 0) ok = false;
+            if (dry_fast[i] == 0 || dry_fast[i] == 6) ok = false;
             if (dry_passes[i].fused && dry_fast[i] != 5) ok = false;
         }
         dry_passes.clear();
@@ -537,9 +538,241 @@ MultSpec Solver::mult_spec(int type) const {
     return G;
 }
 
-// Which register-resident kernel can run this pass (0 = none: the general line pass).
+// Which kernel runs this pass: a register DFT (1-5), the mixed-radix pass (6),
+// or the general line pass (0).
 int Solver::fast_kind(const PassArgs& A, bool f64, bool in_f64, bool out_f64) const {
     if (!use_fast) return 0;
+    if (const int k = reg_kind(A, f64, in_f64, out_f64)) return k;
+    return use_mix && mix_op(A, f64, in_f64, out_f64) >= 0 ? 6 : 0;
+}
+
+// r2r kinds: FFTW's type (1-4) and whether it is the odd one; type 0 for others
+static int r2r_type(int kind) {
+    if (kind >= LK_DCT1 && kind <= LK_DCT4) return kind - LK_DCT1 + 1;
+    if (kind >= LK_DST1 && kind <= LK_DST4) return kind - LK_DST1 + 1;
+    return 0;
+}
+static bool r2r_odd(int kind) { return kind >= LK_DST1 && kind <= LK_DST4; }
+
+// points of the complex transform of a mixed-radix pass
+static int mix_length(const LineStage& S) {
+    const LineSpec& sp = S.spec[0];
+    switch (r2r_type(sp.kind)) {
+        case 2: case 3: return sp.n_in;
+        case 4: return sp.n_in % 2 == 0 ? sp.n_in / 2 : 0;
+    }
+    return S.M;
+}
+
+// The mixed-radix pass that can run this pass (MixOp), or -1.  It takes what
+// the register DFTs leave: any length with prime factors up to 13 that splits
+// into two to four stages, any strides and alignment of the real side.  Lines
+// whose output line holds anything but the transform's outputs, zeros set by
+// the plan and the periodic copy stay on the general line pass.
+int Solver::mix_op(const PassArgs& A, bool f64, bool in_f64, bool out_f64) const {
+    const bool rot = A.fused && A.mult.mode == 2;
+    // components together: only the fused ROT pass (the curl tables exist once set up; host-only planning assumes them)
+    if (rot != (A.comps_together != 0) || (rot && (A.lda != 3 || A.ncomp != 3 || !(ksym || dry)))) return -1;
+    if (A.n_b > 65535 || A.ncomp > 65535) return -1;
+    const LineStage& S = A.st[0];
+    const LineStage& E = A.st[A.fused ? 1 : 0];  // the stage that stores
+    const int k0 = S.spec[0].kind, t0 = r2r_type(k0), t1 = r2r_type(E.spec[0].kind);
+    const bool period = t1 == 0 && E.spec[0].postpro == PP_ENFORCE_PERIOD;
+    for (int s2 = 0; s2 <= A.fused; ++s2) {
+        const LineStage& X = A.st[s2];
+        const LineSpec& x0 = X.spec[0];
+        const int type = r2r_type(x0.kind);
+        for (int c = 0; c < A.lda; ++c) {
+            const LineSpec& sp = X.spec[c];
+            if (type == 0) {
+                if (sp.kind != x0.kind || sp.n_in != x0.n_in || sp.fi != 0 || sp.fo != 0 || sp.postpro != x0.postpro ||
+                    (sp.postpro == PP_ENFORCE_PERIOD && sp.nfftw != x0.nfftw))
+                    return -1;
+                if (sp.postpro != PP_NONE && sp.postpro != PP_ENFORCE_PERIOD) return -1;
+            } else {
+                if (r2r_type(sp.kind) != type || (sp.postpro & PP_ENFORCE_PERIOD) || (type != 1 && sp.n_in != x0.n_in)) return -1;
+                // every stored element outside the transform is a zero of the plan, and no zero lies inside
+                const bool first = sp.postpro & PP_NULL_FIRST, last = sp.postpro & PP_NULL_LAST;
+                const int lo = sp.fo, hi = sp.fo + sp.n_in;
+                if ((first && lo == 0) || (last && X.n_o - 1 >= lo && X.n_o - 1 < hi)) return -1;
+                if (s2 == A.fused) {
+                    for (int i = X.store_off; i < X.store_off + X.n_store; ++i) {
+                        if (i >= lo && i < hi) i = hi - 1;
+                        else if (!(first && i == 0) && !(last && i == X.n_o - 1)) return -1;
+                    }
+                }
+                if (s2 == 1 && (sp.fi != S.spec[c].fo || sp.n_in != S.spec[c].n_in || r2r_odd(sp.kind) != r2r_odd(S.spec[c].kind)))
+                    return -1;
+            }
+        }
+        if (type == 0 && (X.fieldstart != 0 || X.store_off != 0)) return -1;
+    }
+    const int M = mix_length(S);
+    int op = -1, full = M;  // outputs the transform itself gives
+    if (A.fused) {
+        if ((A.mult.mode != 1 && !rot) || A.in != A.out || A.in_cstr != A.out_cstr) return -1;
+        for (int d = 0; d < 3; ++d)
+            if (A.in_str[d] != A.out_str[d]) return -1;
+        const int k1 = E.spec[0].kind, fold = A.mult.gfold[A.axis];
+        if (k0 == LK_C2C && k1 == LK_C2C && E.M == M && S.spec[0].sign < 0 && E.spec[0].sign > 0 && fold == M)
+            op = rot ? MX_ROT : MX_FUSED;
+        else if (rot) return -1;
+        else if (k0 == LK_R2C && k1 == LK_C2R && E.M == M && fold == 0) op = MX_FUSED_R;
+        else if (t0 == 2 && t1 == 3 && fold == 0) op = MX_FUSED_23;
+        else if (t0 == 3 && t1 == 2 && fold == 0) op = MX_FUSED_32;
+        else if (t0 == 1 && t1 == 1 && fold == 0) op = MX_FUSED_11;
+        else if (t0 == 4 && t1 == 4 && fold == 0) op = MX_FUSED_44;
+        if (op < 0 || (int64_t)(S.n_o + 1) * A.mult.gstr[A.axis] >= (int64_t)INT32_MAX) return -1;
+    } else if (k0 == LK_C2C) {
+        op = S.spec[0].sign > 0 ? MX_C2C_I : MX_C2C_F;
+    } else if (k0 == LK_R2C) {
+        op = MX_R2C;
+        full = M / 2 + 1;
+    } else if (k0 == LK_C2R) {
+        op = MX_C2R;
+        if (A.n_src < M / 2 + 1) return -1;
+    } else {
+        const int ops[5] = {-1, MX_T1, MX_T2, MX_T3, MX_T4};
+        op = ops[t0];
+    }
+    if (op < 0) return -1;
+    // the stored line: the transform's outputs and at most the periodic copy after them
+    if (t1 == 0 && (E.n_store > full + (period ? 1 : 0) || (period && (E.n_store != full + 1 || E.spec[0].nfftw != full)))) return -1;
+    const bool rin = k0 == LK_R2C || t0 != 0, rout = E.spec[0].kind == LK_C2R || t1 != 0;
+    if (S.in_cplx == (rin ? 1 : 0) || E.out_cplx == (rout ? 1 : 0)) return -1;
+    if (rin && !A.fused ? (f64 && !in_f64) : in_f64 != f64) return -1;
+    if (rout && !A.fused ? (f64 && !out_f64) : out_f64 != f64) return -1;
+    const int64_t n = std::max(std::max(A.n_src, E.n_store), S.M) + 1;
+    if (n * A.in_str[A.axis] >= (int64_t)INT32_MAX || n * A.out_str[A.axis] >= (int64_t)INT32_MAX) return -1;
+    const uintptr_t ain = dry ? 0 : (uintptr_t)A.in, aout = dry ? 0 : (uintptr_t)A.out;
+    const uintptr_t cb = f64 ? 16 : 8;
+    if (ain % (rin ? (in_f64 ? 8 : 4) : cb) != 0 || aout % (rout ? (out_f64 ? 8 : 4) : cb) != 0) return -1;
+    return M > 0 && mix_plan_of(M, op, f64) ? op : -1;
+}
+
+// the factorisation of a length, searched once per solver; nullptr: none
+const MixPlan* Solver::mix_plan_of(int M, int op, bool f64) const {
+    const std::array<int, 3> key{M, op, f64 ? 1 : 0};
+    auto it = mix_plans.find(key);
+    if (it == mix_plans.end()) {
+        MixPlan p{};
+        if (!mix_plan(M, op, f64 ? 1 : 0, p) || !mix_fits(p, op, f64 ? 1 : 0)) p.ns = 0;
+        it = mix_plans.emplace(key, p).first;
+    }
+    return it->second.ns ? &it->second : nullptr;
+}
+
+// arguments of a mixed-radix launch, all but the twiddles
+void Solver::mix_args(const PassArgs& A, int op, bool f64, bool in_f64, bool out_f64, MixArgs& m) const {
+    const LineStage& E = A.st[A.fused ? 1 : 0];
+    const int a = (A.axis == 0) ? 1 : 0, b = (A.axis == 2) ? 1 : 2;
+    memset(&m, 0, sizeof(m));
+    m.in = A.in;
+    m.out = A.out;
+    m.na = A.n_a;
+    m.nb = A.n_b;
+    m.n_src = A.n_src;
+    m.n_store = E.n_store;
+    m.in_sl = A.in_str[A.axis];
+    m.in_sa = A.in_str[a];
+    m.in_sb = A.in_str[b];
+    m.in_sc = A.in_cstr;
+    m.out_sl = A.out_str[A.axis];
+    m.out_sa = A.out_str[a];
+    m.out_sb = A.out_str[b];
+    m.out_sc = A.out_cstr;
+    m.in64 = in_f64;
+    m.out64 = out_f64;
+    m.period = op < MX_T2 || op == MX_FUSED_R ? (E.spec[0].postpro == PP_ENFORCE_PERIOD ? E.spec[0].nfftw : -1) : -1;
+    m.fieldstart = A.st[0].fieldstart;
+    m.store_off = E.store_off;
+    m.lda = A.lda;
+    for (int c = 0; c < 3; ++c) {
+        const LineSpec &x = A.st[0].spec[c], &y = E.spec[c];
+        m.N[c] = x.n_in;
+        m.dst[c] = r2r_odd(x.kind);
+        m.fi[c] = x.fi;
+        m.fo[c] = y.fo;
+        m.go[c] = x.fo;
+        m.z0[c] = (op >= MX_T2 && op != MX_FUSED_R && (y.postpro & PP_NULL_FIRST) && E.store_off == 0) ? 0 : -1;
+        const int last = E.n_o - 1 - E.store_off;
+        m.z1[c] = (op >= MX_T2 && op != MX_FUSED_R && (y.postpro & PP_NULL_LAST) && last >= 0 && last < E.n_store) ? last : -1;
+    }
+    if (A.fused) {
+        m.green = A.mult.green;
+        m.g_sa = A.mult.gstr[a];
+        m.g_sb = A.mult.gstr[b];
+        m.g_sl = A.mult.gstr[A.axis];
+        m.f_a = A.mult.gfold[a];
+        m.f_b = A.mult.gfold[b];
+        m.f_l = A.mult.gfold[A.axis];
+    }
+    if (op == MX_ROT) {
+        m.ksym = ksym;
+        m.kstr = kstr;
+        m.ax_a = a;
+        m.ax_b = b;
+        m.ax_l = A.axis;
+    }
+    m.pl = *mix_plan_of(mix_length(A.st[0]), op, f64);
+    // the tile depends on the extents only: searched once per solver
+    const std::array<int, 7> key{m.pl.M, op, f64 ? 1 : 0, A.axis == 0 ? 1 : 0, A.n_a, A.n_b, A.ncomp};
+    auto it = mix_tiles.find(key);
+    if (it == mix_tiles.end()) {
+        mix_tile(m, f64 ? 1 : 0, op, A.axis == 0, A.ncomp / mix_planes(op));
+        it = mix_tiles.emplace(key, std::array<int, 2>{m.tx, m.P}).first;
+    }
+    m.tx = it->second[0];
+    m.P = it->second[1];
+}
+
+const void* Solver::mix_table(const MixPlan& p, bool f64) {
+    int64_t key = ((int64_t)1 << 50) + ((int64_t)p.M << 20) + (f64 ? 1 : 0);
+    for (int s = 0; s < p.ns; ++s) key += (int64_t)(p.st[s].R - 1) << (4 + 4 * s);
+    auto it = twiddles.find(key);
+    if (it != twiddles.end()) return it->second;
+    std::vector<double> w(2 * (size_t)std::max(p.ntw, 1), 0.0);
+    for (int e = 0; e < p.ntw; ++e) {
+        int q = 0, n = 1;
+        mix_twiddle_exponent(p, e, &q, &n);
+        const long double a = -2.0L * (long double)M_PI * (long double)q / (long double)n;
+        w[2 * e] = (double)cosl(a);
+        w[2 * e + 1] = (double)sinl(a);
+    }
+    return twiddles[key] = upload_table(w, f64);
+}
+
+// W_8N^{4j+1}, j < N/2: the pre-twiddles of the type-IV kinds
+const void* Solver::type4_table(int N, bool f64) {
+    const int64_t key = ((int64_t)1 << 51) + (int64_t)N * 2 + (f64 ? 1 : 0);
+    auto it = twiddles.find(key);
+    if (it != twiddles.end()) return it->second;
+    std::vector<double> w(2 * (size_t)(N / 2));
+    for (int j = 0; j < N / 2; ++j) {
+        const long double a = -2.0L * (long double)M_PI * (long double)(4 * j + 1) / (8.0L * (long double)N);
+        w[2 * j] = (double)cosl(a);
+        w[2 * j + 1] = (double)sinl(a);
+    }
+    return twiddles[key] = upload_table(w, f64);
+}
+
+// device copy of a table of complex values, in the working precision
+void* Solver::upload_table(const std::vector<double>& w, bool f64) {
+    void* d = nullptr;
+    if (f64) {
+        check_cuda(cudaMalloc(&d, w.size() * sizeof(double)), "twiddle allocation");
+        check_cuda(cudaMemcpy(d, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice), "twiddle upload");
+    } else {
+        std::vector<float> wf(w.size());
+        for (size_t i = 0; i < w.size(); ++i) wf[i] = (float)w[i];
+        check_cuda(cudaMalloc(&d, wf.size() * sizeof(float)), "twiddle allocation");
+        check_cuda(cudaMemcpy(d, wf.data(), wf.size() * sizeof(float), cudaMemcpyHostToDevice), "twiddle upload");
+    }
+    return d;
+}
+
+// Which register-resident kernel can run this pass (0 = none).
+int Solver::reg_kind(const PassArgs& A, bool f64, bool in_f64, bool out_f64) const {
     // components together: only the fused ROT pass (groups of three components)
     const bool rot = A.fused && A.mult.mode == 2;
     // (the curl tables exist once set up; host-only planning assumes them)
@@ -771,6 +1004,19 @@ void Solver::rowfused_args(const PassArgs& A, RowFusedArgs& f) const {
 
 void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, bool out_f64) {
     const int L = A.st[0].M;
+    if (kind == 6) {
+        MixArgs m;
+        const int op = mix_op(A, f64, in_f64, out_f64);
+        mix_args(A, op, f64, in_f64, out_f64, m);
+        m.tw = mix_table(m.pl, f64);
+        if (mix_mirrors(op) && op >= MX_T2 && op != MX_FUSED_R) m.tw4 = twiddle(2 * m.N[0], f64);
+        if (op == MX_T4 || op == MX_FUSED_44) {
+            m.tw4 = twiddle(2 * m.N[0], f64);
+            m.tw8 = type4_table(m.N[0], f64);
+        }
+        check_cuda(launch_mix(f64 ? 1 : 0, op, A.axis == 0, m, A.ncomp, stream), "mixed-radix pass launch");
+        return;
+    }
     if (kind == 5) {
         RowFusedArgs f;
         rowfused_args(A, f);
@@ -965,8 +1211,9 @@ void Solver::run_pass(const PassArgs& Ain, bool f64, bool in_f64, bool out_f64, 
     // a connected share's y passes must reach the owners' column arrays
     FLB_CHECK(!(peers.n > 0 && owned() && slab_dim == 2 && A.axis == 1 && !A.fused) || (fk == 1 && A.ncomp == 1),
               "a share connected to its peers' column arrays needs register-DFT y passes");
-    for (int s2 = 0; s2 <= A.fused; ++s2)
-        if (!A.st[s2].tw) A.st[s2].tw = twiddle(A.st[s2].M, f64);
+    if (fk == 0)
+        for (int s2 = 0; s2 <= A.fused; ++s2)
+            if (!A.st[s2].tw) A.st[s2].tw = twiddle(A.st[s2].M, f64);
     // algorithmic bytes: source and kept output lines once, the folded Green's spectrum once
     const int64_t nc = A.ncomp;
     const double es = f64 ? 8.0 : 4.0;
@@ -1192,7 +1439,12 @@ void Solver::compute_green() {
         A.in = gb[cb];
         A.out = gb[1 - cb];
         fit_lines(A, sizeof(double));
+        // one line per complex transform: a pair's rounding would put the
+        // line next to the origin's peak into its neighbour
+        const bool keep_mix = use_mix;
+        use_mix = false;
         run_pass(A, true, true, true, "green");
+        use_mix = keep_mix;
         cb = 1 - cb;
         cur = nxt;
     }
