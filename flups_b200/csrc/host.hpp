@@ -227,8 +227,8 @@ struct Solver {
     const void* mix_table(const flb::MixPlan& p, bool f64);
     const void* type4_table(int N, bool f64);
     void* upload_table(const std::vector<double>& w, bool f64);
-    const flb::MixPlan* mix_plan_of(int M, int op, bool f64) const;
-    mutable std::map<std::array<int, 3>, flb::MixPlan> mix_plans;         // per length, operation and precision
+    const flb::MixPlan* mix_plan_of(int M, int op, bool rows, bool f64) const;
+    mutable std::map<std::array<int, 4>, flb::MixPlan> mix_plans;         // per length, operation, rows and precision
     mutable std::map<std::array<int, 7>, std::array<int, 2>> mix_tiles;   // and per extents: lines, threads per line
     bool use_mix = true;                  // false while the no-allocation solve plans its passes
     // arguments of a fast launch, all but the twiddle tables; mode of a column pass

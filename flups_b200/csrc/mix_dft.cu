@@ -9,23 +9,21 @@ namespace flb {
 
 namespace {
 
-constexpr int kRadices[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 15, 16};
-
-// radices of a last stage that takes two or three butterflies in one thread
-bool small_radix(int r) { return r <= 8 || r == 11 || r == 13; }
+// the last stage takes the butterflies of k and M - k, or of three components, together
+bool small_last(int op) { return mix_mirrors(op) || op == MX_ROT; }
 
 // search over ordered factorisations: fewest stages first (each one is a
 // round trip through shared memory), then the smallest sum of the radices
-// (butterfly work), then the larger radix first
+// (butterfly work), then the order with the larger radices first
 struct Search {
-    int op, f64;
+    int op, cls;
+    bool f64;
     int best[kMixStages], nbest = 0, cost = 1 << 30;
     int cur[kMixStages];
     void go(int m, int n, int sum) {
         if (m == 1) {
-            if (n < 2) return;
-            if ((mix_mirrors(op) || op == MX_ROT) && !small_radix(cur[n - 1])) return;
-            int up = 0;  // steps up: the order with the larger radices first wins
+            if (n < 2 || (small_last(op) && !mix_radix_ok(cls, f64, true, cur[n - 1]))) return;
+            int up = 0;
             for (int i = 1; i < n; ++i) up += cur[i] > cur[i - 1];
             const int c = n * 10000 + sum * 100 + up;
             if (c < cost) {
@@ -35,27 +33,59 @@ struct Search {
             }
             return;
         }
-        if (n == kMixStages) return;
-        for (int r : kRadices) {
-            if (m % r != 0 || r > max_radix()) continue;
+        if (n == (cls == MIX_TWO ? 2 : kMixStages)) return;
+        for (int r = 2; r <= 32; ++r) {
+            // (a small last radix need not be one of the others)
+            if (m % r != 0 || !(mix_radix_ok(cls, f64, false, r) || (m == r && small_last(op)))) continue;
             cur[n] = r;
             go(m / r, n + 1, sum + r);
         }
     }
-    // FP64 butterflies of 15 and 16 values do not fit the 128 registers of two CTAs per SM
-    int max_radix() const { return f64 ? 13 : 16; }
 };
+
+int host_block(const MixPlan& p, int s, int q) {
+    int off = q % p.st[0].R * p.s1, k = q / p.st[0].R;
+    for (int i = 1; i < s; ++i) {
+        off += k % p.st[i].R * p.st[i].nn;
+        k /= p.st[i].R;
+    }
+    return off;
+}
+
+// shared-memory cycles of a row tile's accesses after the first stage: lanes
+// along a line, `lanes` of them per cycle when their banks differ
+int row_cycles(const MixPlan& p, int lanes) {
+    int total = 0;
+    for (int s = 1; s < p.ns; ++s) {
+        const int nb = p.st[s].nn * p.st[s].Q;
+        for (int b0 = 0; b0 < nb; b0 += lanes) {
+            int hits[16] = {0}, worst = 0;
+            for (int b = b0; b < std::min(nb, b0 + lanes); ++b) {
+                const int m = b / p.st[s].Q;
+                worst = std::max(worst, ++hits[(host_block(p, s, b - m * p.st[s].Q) + m) % lanes]);
+            }
+            total += worst * p.st[s].R;
+        }
+    }
+    return total;
+}
 
 }  // namespace
 
-bool mix_plan(int M, int op, int f64, MixPlan& p) {
+bool mix_plan(int M, int op, bool rows, int f64, MixPlan& p) {
     if (M < 4 || M > 16384) return false;
-    Search s{op, f64};
+    Search s{op, MIX_MULTI, f64 != 0};
     s.go(M, 0, 0);
+    if (s.nbest != 2 && mix_two(op, rows)) {
+        Search t{op, MIX_TWO, f64 != 0};
+        t.go(M, 0, 0);
+        if (t.nbest) s = t;
+    }
     if (s.nbest == 0) return false;
     p = MixPlan{};
     p.M = M;
     p.ns = s.nbest;
+    p.cls = s.cls;
     int Q = 1, left = M;
     for (int i = 0; i < s.nbest; ++i) {
         MixStage& st = p.st[i];
@@ -68,7 +98,22 @@ bool mix_plan(int M, int op, int f64, MixPlan& p) {
         if (i + 1 < s.nbest) p.ntw += (st.R - 1) * left;
         Q *= st.R;
     }
+    // columns: an odd distance puts the rows met by a half-warp on distinct
+    // banks; rows: the distance of the fewest shared-memory cycles
     p.s1 = p.st[0].nn | 1;
+    if (rows) {
+        const int lanes = f64 ? 8 : 16;
+        int best = 1 << 30, at = p.s1;
+        for (int d = 0; d < lanes; ++d) {
+            p.s1 = p.st[0].nn + d;
+            const int c = row_cycles(p, lanes);
+            if (c < best) {
+                best = c;
+                at = p.s1;
+            }
+        }
+        p.s1 = at;
+    }
     p.len = p.st[0].R * p.s1;
     return true;
 }
@@ -82,58 +127,64 @@ void mix_twiddle_exponent(const MixPlan& p, int e, int* q, int* n) {
     *n = st.R * st.nn;
 }
 
-// lines per CTA and threads per line.  Shared memory for three resident CTAs
-// where the line allows it, 256 threads at most; the number of threads per line
-// wastes the fewest butterfly slots over the stages.
+// lines per CTA and threads per line: the tile of the least cost, a product of
+//  - butterfly slots offered over those needed, whole warps counted,
+//  - the column tile's run of x: 128 bytes 1, 64 bytes 1.15, 32 bytes 1.35
+//    (400-point fused columns at 200^3, FP32: 156 us with 16 columns, 170 with
+//    8; FP64: 302 with 8, 354 with 4),
+//  - small against large CTAs: 128 to 160 threads ran best (several resident
+//    CTAs overlap one's barriers with another's loads; 240 points FP32: 41 us
+//    with 128 threads, 46 with 256),
+//  - too few resident threads (shared memory, registers), and too few CTAs for
+//    the 148 SMs.
 void mix_tile(MixArgs& a, int f64, int op, bool rows, int64_t ncomp) {
-    const bool pair = mix_pairs(op);
     const size_t line = (size_t)a.pl.len * mix_planes(op) * (f64 ? 16 : 8);
-    const int64_t lines = (int64_t)mix_units(a.na, pair, rows) * (rows ? a.nb : 1);
+    const int64_t lines = (int64_t)mix_units(a.na, mix_pairs(op), rows) * (rows ? a.nb : 1);
     const int64_t outer = (rows ? 1 : (int64_t)a.nb) * ncomp;
-    const size_t target = 72 * 1024;
-    int maxp = 1, minnb = 1 << 30;
-    for (int s = 0; s < a.pl.ns; ++s) {
-        const int nb = a.pl.M / a.pl.st[s].R;
-        maxp = std::max(maxp, nb);
-        minnb = std::min(minnb, nb);
-    }
-    auto waste = [&](int P, int tx) {
-        // butterfly slots offered over those needed
+    const int maxth = mix_threads(f64, a.pl.cls);
+    int maxp = 1;
+    for (int s = 0; s < a.pl.ns; ++s) maxp = std::max(maxp, a.pl.M / a.pl.st[s].R);
+    // registers per thread of the kernel, and the resident threads per SM that hide its latencies
+    const int regs = a.pl.cls == MIX_TWO ? (f64 ? 168 : 128) : (f64 ? 128 : 80), want = f64 ? 384 : 480;
+    double best = 1e30;
+    a.tx = 1;
+    a.P = std::min(maxp, 32);
+    auto consider = [&](int tx, int P) {
+        const size_t smem = tx * line;
+        if (smem > 227 * 1024) return;
         double need = 0, have = 0;
         for (int s = 0; s < a.pl.ns; ++s) {
             const int nb = a.pl.M / a.pl.st[s].R;
-            need += nb * (double)a.pl.st[s].R;
+            need += (double)nb * a.pl.st[s].R;
             have += (double)((nb + P - 1) / P) * P * a.pl.st[s].R;
         }
-        const int th = P * tx, up = (th + 31) / 32 * 32;
-        return have / need * up / th;
-    };
-    a.tx = 1;
-    a.P = std::min(maxp, 32);
-    double cost = 1e30;
-    auto consider = [&](int tx, int P) {
-        const double c = waste(P, tx) * (1.0 + 24.0 / (P * tx));
-        if (c < cost) {
-            cost = c;
+        const int th = P * tx;
+        double c = have / need * ((th + 31) / 32 * 32) / th * (1.0 + 10.0 / th + std::max(0, th - 160) * 0.001);
+        if (!rows) {
+            const int run = tx * (f64 ? 16 : 8);
+            c *= run >= 128 ? 1.0 : (run >= 96 ? 1.03 : (run >= 64 ? 1.15 : (run >= 32 ? 1.35 : 1.8)));
+        }
+        const int ctas_sm = std::min((int)(227 * 1024 / (smem + 1024)), 65536 / (regs * ((th + 31) / 32 * 32)));
+        const int resident = std::max(1, ctas_sm) * th;
+        if (resident < want) c *= 1.0 + 0.5 * ((double)want / resident - 1.0);
+        const double ctas = (double)((lines + tx - 1) / tx) * outer;
+        if (ctas < 148) c *= 1.3 * 148 / ctas;
+        else if (ctas < 296) c *= 1.0 + 0.3 * (296 - ctas) / 148;
+        if (c < best) {
+            best = c;
             a.tx = tx;
             a.P = P;
         }
     };
     if (rows) {
-        for (int P = std::min(16, maxp); P <= std::min(maxp, kMixThreads); ++P) {
-            for (int tx = std::max(1, kMixThreads / P); tx >= 1; --tx) {
-                if (tx > 1 && (size_t)tx * line > target) continue;
-                if (tx > 1 && (lines + tx - 1) / tx * outer < 296) continue;  // two CTAs per SM before larger tiles
-                consider(tx, P);
-            }
-        }
+        for (int P = std::min(16, maxp); P <= std::min(maxp, maxth); ++P)
+            for (int tx = std::max(1, maxth / P); tx >= 1; --tx) consider(tx, P);
         return;
     }
-    int tx = f64 ? 4 : 8;
-    while (tx > 2 && ((size_t)tx * line > target || (lines + tx - 1) / tx * outer < 296)) tx /= 2;
-    if ((size_t)tx * line > 227 * 1024) tx = 1;
-    for (int P = std::max(1, std::min(maxp, 32 / tx)); P <= std::min(maxp, kMixThreads / tx); ++P) {
-        consider(tx, P);
+    for (int run : {16, 12, 8, 6, 4, 2, 1}) {
+        const int tx = f64 ? (run == 1 ? 0 : run / 2) : run;
+        if (tx == 0) continue;
+        for (int P = 1; P <= std::min(maxp, maxth / tx); ++P) consider(tx, P);
     }
 }
 

@@ -37,7 +37,30 @@ constexpr bool mix_mirrors(int op) {
 }
 
 constexpr int kMixStages = 4;
-constexpr int kMixThreads = 256;
+// kernel classes: two to four stages of smaller radices, or two of larger ones
+enum MixClass : int { MIX_MULTI = 0, MIX_TWO = 1 };
+constexpr int mix_threads(int f64, int cls) { return cls == MIX_TWO && f64 ? 128 : 256; }
+// the operations compiled in class TWO: column passes (row passes lose by it:
+// 288-point real rows of a 145 x 121 x 101 grid, FP32, 20 us in 9 x 8 x 4, 26
+// us in 18 x 16; their lanes already run along the line, so fewer threads
+// share it)
+constexpr bool mix_two(int op, bool rows) {
+    return !rows && (op == MX_R2C || op == MX_C2R || op == MX_C2C_F || op == MX_C2C_I || op == MX_FUSED);
+}
+// radices of a class.  small: of a last stage that takes two or three
+// butterflies in one thread.  The limits are those that keep the butterflies
+// in the class's registers.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr bool mix_radix_ok(int cls, bool f64, bool small, int r) {
+    if (cls == MIX_TWO) {
+        if (small) return r >= 4 && r <= (f64 ? 10 : 12);
+        return (r >= 8 && r <= 16) || r == 18 || r == 20 || (!f64 && (r == 24 || r == 25 || r == 32));
+    }
+    if (small) return (r >= 2 && r <= 8) || r == 11 || r == 13;
+    return r >= 2 && r != 14 && r <= (f64 ? 13 : 16);
+}
 
 // Stage s of the decimation in frequency: radix R on sub-blocks of R * nn
 // points (nn points are left of each after it); Q = product of the radices
@@ -49,8 +72,8 @@ struct MixStage {
 };
 
 struct MixPlan {
-    int M, ns;              // line length, number of stages
-    int s1;                 // distance in shared memory between the first digit's blocks (odd)
+    int M, ns, cls;         // line length, number of stages, kernel class
+    int s1;                 // distance in shared memory between the first digit's blocks
     int len;                // elements a line takes in shared memory
     int ntw;                // complex entries of the stage twiddles
     MixStage st[kMixStages];
@@ -86,7 +109,7 @@ struct MixArgs {
 
 // Factorisation of M for a pass of operation `op`; false when M has a prime
 // factor above 13, or does not split into two to four of the radices.
-bool mix_plan(int M, int op, int f64, MixPlan& p);
+bool mix_plan(int M, int op, bool rows, int f64, MixPlan& p);
 // W_{R nn}^{k m} of entry e of the stage twiddles: exponent and root order
 void mix_twiddle_exponent(const MixPlan& p, int e, int* q, int* n);
 // lines per CTA and threads per line (a.tx, a.P) for the pass's extents

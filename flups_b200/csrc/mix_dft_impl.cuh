@@ -31,11 +31,16 @@
 
 namespace flb {
 
-// CTAs per SM the compiler is asked for: three of 256 threads in FP32 (80
-// registers), two in FP64 (128)
-template <typename T> struct MixOcc {
-    static constexpr int threads = kMixThreads;
-    static constexpr int blocks = sizeof(T) == 8 ? 2 : 3;
+// Two classes of kernels.  MULTI: two to four stages of radices up to 16,
+// three 256-thread CTAs per SM in FP32 (80 registers), two in FP64 (128).
+// TWO: exactly two stages, radices up to 32 in FP32 (128 registers, 512
+// threads per SM) and 20 in FP64 (168 registers, 384 threads), for lengths
+// that MULTI runs in three: a stage less is a round trip through shared memory,
+// a twiddle product per value and a barrier less (400-point fused columns of
+// a 200^3 grid, FP32: 10 x 8 x 5 186 us, 20 x 20 156 us; FP64 302 -> 254 us).
+template <typename T, int CLS> struct MixOcc {
+    static constexpr int threads = mix_threads(sizeof(T) == 8, CLS);
+    static constexpr int blocks = CLS == MIX_TWO ? (sizeof(T) == 8 ? 3 : 2) : (sizeof(T) == 8 ? 2 : 3);
 };
 
 // x / d for x d < 2^32, mul = ceil(2^32 / d)
@@ -51,29 +56,18 @@ template <int N, int I = 0, typename F> __device__ __forceinline__ void mix_each
     }
 }
 
-// f with the radix as a compile-time constant.  SMALL: the last stage of a
-// pair, which holds two butterflies
-template <bool SMALL, typename F> __device__ __forceinline__ void mix_radix(int R, F&& f) {
-    switch (R) {
-        case 2: f(MixInt<2>{}); break;
-        case 3: f(MixInt<3>{}); break;
-        case 4: f(MixInt<4>{}); break;
-        case 5: f(MixInt<5>{}); break;
-        case 6: f(MixInt<6>{}); break;
-        case 7: f(MixInt<7>{}); break;
-        case 8: f(MixInt<8>{}); break;
-        case 11: f(MixInt<11>{}); break;
-        case 13: f(MixInt<13>{}); break;
-        default:
-            if constexpr (!SMALL) {
-                switch (R) {
-                    case 9: f(MixInt<9>{}); break;
-                    case 10: f(MixInt<10>{}); break;
-                    case 12: f(MixInt<12>{}); break;
-                    case 15: f(MixInt<15>{}); break;
-                    case 16: f(MixInt<16>{}); break;
-                }
+// f with the radix as a compile-time constant: the radices of a class (F64:
+// of its FP64 kernels); SMALL: of a last stage that holds two or three
+// butterflies
+template <int CLS, bool F64, bool SMALL, int R = 32, typename F> __device__ __forceinline__ void mix_radix(int r, F&& f) {
+    if constexpr (R >= 2) {
+        if constexpr (mix_radix_ok(CLS, F64, SMALL, R)) {
+            if (r == R) {
+                f(MixInt<R>{});
+                return;
             }
+        }
+        mix_radix<CLS, F64, SMALL, R - 1>(r, f);
     }
 }
 
@@ -87,9 +81,10 @@ __device__ __forceinline__ int mix_mirror(int by, int n, int fold) {
     return (by & 1) ? m : n - m;
 }
 
-template <typename T, bool ROWS>
+template <typename T, bool ROWS, int CLS>
 struct MixLine {
     using C = typename CT<T>::C;
+    static constexpr bool F64 = sizeof(T) == 8;
     C* sm;           // element 0 of this thread's line
     int es;          // elements between neighbouring elements of the line
     int p, P;        // this thread of the line's P
@@ -100,7 +95,7 @@ struct MixLine {
     __device__ __forceinline__ int step(int n) const { return ROWS ? n : n * es; }
     // place of the block with digits (k_1, ..., k_{s-1}) packed in q, k_1 fastest (s: stage, from 0)
     __device__ __forceinline__ int block(int s, int q) const {
-        if (s == 1) return q * pl.s1;
+        if (CLS == MIX_TWO || s == 1) return q * pl.s1;
         int k = mix_div(q, pl.st[0].R, pl.st[1].qmul);
         int off = (q - k * pl.st[0].R) * pl.s1;
         if (s == 2) return off + k * pl.st[1].nn;
@@ -109,7 +104,7 @@ struct MixLine {
     }
     // forward first stage: ld(v, m, nn) fills v[n] = x[m + n nn]
     template <typename LD> __device__ __forceinline__ void first(LD&& ld) const {
-        mix_radix<false>(pl.st[0].R, [&](auto rc) {
+        mix_radix<CLS, F64, false>(pl.st[0].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int nn = pl.st[0].nn, d = step(pl.s1);
             for (int m = p; m < nn; m += P) {
@@ -126,7 +121,7 @@ struct MixLine {
     }
     // forward middle stage
     __device__ __forceinline__ void middle(int s) const {
-        mix_radix<false>(pl.st[s].R, [&](auto rc) {
+        mix_radix<CLS, F64, false>(pl.st[s].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int nn = pl.st[s].nn, Q = pl.st[s].Q, d = step(nn);
             for (int b = p; b < nn * Q; b += P) {
@@ -145,7 +140,7 @@ struct MixLine {
     }
     // inverse middle stage
     __device__ __forceinline__ void middle_inv(int s) const {
-        mix_radix<false>(pl.st[s].R, [&](auto rc) {
+        mix_radix<CLS, F64, false>(pl.st[s].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int nn = pl.st[s].nn, Q = pl.st[s].Q, d = step(nn);
             for (int b = p; b < nn * Q; b += P) {
@@ -164,7 +159,7 @@ struct MixLine {
     }
     // inverse last stage: st(v, m, nn) stores v[n] = x[m + n nn]
     template <typename ST> __device__ __forceinline__ void first_inv(ST&& sto) const {
-        mix_radix<false>(pl.st[0].R, [&](auto rc) {
+        mix_radix<CLS, F64, false>(pl.st[0].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int nn = pl.st[0].nn, d = step(pl.s1);
             for (int m = p; m < nn; m += P) {
@@ -180,12 +175,14 @@ struct MixLine {
         });
     }
     __device__ __forceinline__ void forward_middles() const {
+        if constexpr (CLS == MIX_TWO) return;
         for (int s = 1; s + 1 < pl.ns; ++s) {
             middle(s);
             __syncthreads();
         }
     }
     __device__ __forceinline__ void inverse_middles() const {
+        if constexpr (CLS == MIX_TWO) return;
         for (int s = pl.ns - 2; s > 0; --s) {
             middle_inv(s);
             __syncthreads();
@@ -237,14 +234,14 @@ struct MixPos {
     }
 };
 
-template <typename T, int OP, bool ROWS>
-__global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_kernel(const __grid_constant__ MixArgs a) {
+template <typename T, int OP, bool ROWS, int CLS>
+__global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::blocks) mix_kernel(const __grid_constant__ MixArgs a) {
     using C = typename CT<T>::C;
     constexpr bool PAIR = mix_pairs(OP);
     extern __shared__ __align__(16) unsigned char smraw[];
     const int c = ROWS ? threadIdx.y : threadIdx.x;  // line of the tile
     const int TX = ROWS ? blockDim.y : blockDim.x;
-    const MixLine<T, ROWS> L{reinterpret_cast<C*>(smraw) + (ROWS ? c * a.pl.len : c), TX, (int)(ROWS ? threadIdx.x : threadIdx.y),
+    const MixLine<T, ROWS, CLS> L{reinterpret_cast<C*>(smraw) + (ROWS ? c * a.pl.len : c), TX, (int)(ROWS ? threadIdx.x : threadIdx.y),
                              (int)(ROWS ? blockDim.x : blockDim.y), a.pl, reinterpret_cast<const C*>(a.tw)};
     const int M = a.pl.M, ns = a.pl.ns;
     const MixPos<PAIR, ROWS> W(a, c, TX, OP == MX_FUSED);
@@ -293,7 +290,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_ker
     if constexpr (OP == MX_C2C_F) {
         C* out = W.template dst<C>(a, 0);
         const int n_store = ok[0] ? (a.n_store < M ? a.n_store : M) : 0;
-        mix_radix<false>(a.pl.st[ns - 1].R, [&](auto rc) {
+        mix_radix<CLS, sizeof(T) == 8, false>(a.pl.st[ns - 1].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int d = L.step(1);
             for (int q = L.p; q < nq; q += L.P) {
@@ -315,7 +312,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_ker
     if constexpr (OP == MX_C2C_I) {
         const C* in = W.template src<C>(a, 0);
         const int n_src = ok[0] ? a.n_src : 0;
-        mix_radix<false>(a.pl.st[ns - 1].R, [&](auto rc) {
+        mix_radix<CLS, sizeof(T) == 8, false>(a.pl.st[ns - 1].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int d = L.step(1);
             for (int q = L.p; q < nq; q += L.P) {
@@ -335,7 +332,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_ker
     if constexpr (OP == MX_FUSED) {
         const T* g = W.template green<T>(a, 0);
         const int gl = (int)a.g_sl;
-        mix_radix<false>(a.pl.st[ns - 1].R, [&](auto rc) {
+        mix_radix<CLS, sizeof(T) == 8, false>(a.pl.st[ns - 1].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int d = L.step(1);
             for (int q = L.p; q < nq; q += L.P) {
@@ -358,7 +355,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_ker
     if constexpr (OP == MX_R2C) {
         C* out0 = W.template dst<C>(a, 0);
         C* out1 = W.template dst<C>(a, 1);
-        mix_radix<true>(a.pl.st[ns - 1].R, [&](auto rc) {
+        mix_radix<CLS, sizeof(T) == 8, true>(a.pl.st[ns - 1].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int d = L.step(1);
             for (int q = L.p; 2 * q <= nq; q += L.P) {
@@ -402,7 +399,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_ker
     if constexpr (OP == MX_C2R) {
         const C* in0 = W.template src<C>(a, 0);
         const C* in1 = W.template src<C>(a, 1);
-        mix_radix<true>(a.pl.st[ns - 1].R, [&](auto rc) {
+        mix_radix<CLS, sizeof(T) == 8, true>(a.pl.st[ns - 1].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int d = L.step(1);
             for (int q = L.p; 2 * q <= nq; q += L.P) {
@@ -492,8 +489,8 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_ker
 // DST-II(x)_k = DCT-II((-1)^j x_j)_{N-1-k}, DST-III(x)_k = (-1)^k DCT-III(x_{N-1-j})_k,
 // DST-IV(x)_k = (-1)^k DCT-IV(x_{N-1-j})_k.  Between type III and type II of
 // a fused pass the two signs cancel.
-template <typename T, int OP, bool ROWS>
-__global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_real_kernel(const __grid_constant__ MixArgs a) {
+template <typename T, int OP, bool ROWS, int CLS>
+__global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::blocks) mix_real_kernel(const __grid_constant__ MixArgs a) {
     using C = typename CT<T>::C;
     constexpr bool PAIR = mix_pairs(OP);
     constexpr bool GREEN = OP >= MX_FUSED_R;
@@ -503,7 +500,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_rea
     extern __shared__ __align__(16) unsigned char smraw[];
     const int c = ROWS ? threadIdx.y : threadIdx.x;
     const int TX = ROWS ? blockDim.y : blockDim.x;
-    const MixLine<T, ROWS> L{reinterpret_cast<C*>(smraw) + (ROWS ? c * a.pl.len : c), TX, (int)(ROWS ? threadIdx.x : threadIdx.y),
+    const MixLine<T, ROWS, CLS> L{reinterpret_cast<C*>(smraw) + (ROWS ? c * a.pl.len : c), TX, (int)(ROWS ? threadIdx.x : threadIdx.y),
                              (int)(ROWS ? blockDim.x : blockDim.y), a.pl, reinterpret_cast<const C*>(a.tw)};
     const MixPos<PAIR, ROWS> W(a, c, TX, GREEN);
     constexpr int H = MixPos<PAIR, ROWS>::H;
@@ -603,7 +600,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_rea
 
     // k and M - k of a pair: f(v, w, q, self, rc) between the forward and / or inverse butterflies of class q and nq - q
     auto mirrored = [&](auto fwd, auto inv, auto&& f) {
-        mix_radix<true>(R_last, [&](auto rc) {
+        mix_radix<CLS, sizeof(T) == 8, true>(R_last, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int d = L.step(1);
             for (int q = L.p; 2 * q <= nq; q += L.P) {
@@ -692,7 +689,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_rea
     }
     if constexpr (OP == MX_T1) {
         with_output([&](auto&& put) {
-            mix_radix<false>(R_last, [&](auto rc) {
+            mix_radix<CLS, sizeof(T) == 8, false>(R_last, [&](auto rc) {
                 constexpr int R = decltype(rc)::v;
                 const int d = L.step(1);
                 for (int q = L.p; q < nq; q += L.P) {
@@ -715,7 +712,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_rea
     }
     if constexpr (OP == MX_T4) {
         with_output([&](auto&& put) {
-            mix_radix<false>(R_last, [&](auto rc) {
+            mix_radix<CLS, sizeof(T) == 8, false>(R_last, [&](auto rc) {
                 constexpr int R = decltype(rc)::v;
                 const int d = L.step(1);
                 for (int q = L.p; q < nq; q += L.P) {
@@ -766,7 +763,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_rea
         });
     }
     if constexpr (OP == MX_FUSED_11 || OP == MX_FUSED_44) {
-        mix_radix<false>(R_last, [&](auto rc) {
+        mix_radix<CLS, sizeof(T) == 8, false>(R_last, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int d = L.step(1);
             for (int q = L.p; q < nq; q += L.P) {
@@ -806,7 +803,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_rea
     __syncthreads();
     L.inverse_middles();
     if constexpr (OP == MX_FUSED_32) {
-        mix_radix<false>(a.pl.st[0].R, [&](auto rc) {
+        mix_radix<CLS, sizeof(T) == 8, false>(a.pl.st[0].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int nn = a.pl.st[0].nn, d = L.step(a.pl.s1);
             for (int m = L.p; m < nn; m += L.P) {
@@ -873,16 +870,16 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_rea
 //   u_g = G (w_{g+2} K_{g+1,g+2} - w_{g+1} K_{g+2,g+1})  (indices mod 3)
 // between the two transforms.  Along the line the symbols change with k;
 // those of the other two directions are constants of the thread.
-template <typename T, bool ROWS>
-__global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_rot_kernel(const __grid_constant__ MixArgs a) {
+template <typename T, bool ROWS, int CLS>
+__global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::blocks) mix_rot_kernel(const __grid_constant__ MixArgs a) {
     using C = typename CT<T>::C;
     extern __shared__ __align__(16) unsigned char smraw[];
     const int c = ROWS ? threadIdx.y : threadIdx.x;
     const int TX = ROWS ? blockDim.y : blockDim.x;
     const int plane = TX * a.pl.len;  // elements of one component's lines
-    const MixLine<T, ROWS> L0{reinterpret_cast<C*>(smraw) + (ROWS ? c * a.pl.len : c), TX, (int)(ROWS ? threadIdx.x : threadIdx.y),
+    const MixLine<T, ROWS, CLS> L0{reinterpret_cast<C*>(smraw) + (ROWS ? c * a.pl.len : c), TX, (int)(ROWS ? threadIdx.x : threadIdx.y),
                               (int)(ROWS ? blockDim.x : blockDim.y), a.pl, reinterpret_cast<const C*>(a.tw)};
-    auto line = [&](int g) { return MixLine<T, ROWS>{L0.sm + g * plane, L0.es, L0.p, L0.P, L0.pl, L0.tw}; };
+    auto line = [&](int g) { return MixLine<T, ROWS, CLS>{L0.sm + g * plane, L0.es, L0.p, L0.P, L0.pl, L0.tw}; };
     const MixPos<false, ROWS> W(a, c, TX, true);
     const int ns = a.pl.ns, nq = a.pl.st[ns - 1].Q;
     const int isl = (int)a.in_sl, osl = (int)a.out_sl;
@@ -921,7 +918,7 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_rot
         }
 #pragma unroll
         for (int e = 0; e < 2; ++e) kl[e] = K + (3 * a.ax_l + (a.ax_l + 1 + e) % 3) * a.kstr;
-        mix_radix<true>(a.pl.st[ns - 1].R, [&](auto rc) {
+        mix_radix<CLS, sizeof(T) == 8, true>(a.pl.st[ns - 1].R, [&](auto rc) {
             constexpr int R = decltype(rc)::v;
             const int d = L0.step(1);
             for (int q = L0.p; q < nq; q += L0.P) {
@@ -978,28 +975,37 @@ __global__ void __launch_bounds__(MixOcc<T>::threads, MixOcc<T>::blocks) mix_rot
     }
 }
 
-template <typename T, int OP, bool ROWS>
+template <typename T, int OP, bool ROWS, int CLS>
 inline cudaError_t launch_mix_t(const MixArgs& a, int ncomp, cudaStream_t s) {
     constexpr bool PAIR = mix_pairs(OP);
     constexpr auto kernel = [] {
-        if constexpr (OP == MX_ROT) return mix_rot_kernel<T, ROWS>;
-        else if constexpr (OP >= MX_T2) return mix_real_kernel<T, OP, ROWS>;
-        else return mix_kernel<T, OP, ROWS>;
+        if constexpr (OP == MX_ROT) return mix_rot_kernel<T, ROWS, CLS>;
+        else if constexpr (OP >= MX_T2) return mix_real_kernel<T, OP, ROWS, CLS>;
+        else return mix_kernel<T, OP, ROWS, CLS>;
     }();
     static std::atomic<unsigned long long> attr{0};
     if (cudaError_t e = smem_attr_once(attr, kernel, 227 * 1024); e != cudaSuccess) return e;
     const int64_t units = (int64_t)mix_units(a.na, PAIR, ROWS) * (ROWS ? a.nb : 1);
     const size_t smem = (size_t)a.tx * a.pl.len * mix_planes(OP) * sizeof(typename CT<T>::C);
-    if (a.tx < 1 || a.P < 1 || a.tx * a.P > kMixThreads || smem > 227 * 1024) return cudaErrorInvalidValue;
+    if (a.tx < 1 || a.P < 1 || a.tx * a.P > MixOcc<T, CLS>::threads || smem > 227 * 1024) return cudaErrorInvalidValue;
     const unsigned gx = (unsigned)((units + a.tx - 1) / a.tx);
     if constexpr (ROWS) kernel<<<dim3(gx, 1, ncomp), dim3(a.P, a.tx), smem, s>>>(a);
     else kernel<<<dim3(gx, a.nb, ncomp), dim3(a.tx, a.P), smem, s>>>(a);
     return cudaGetLastError();
 }
 
+template <typename T, int OP, bool ROWS>
+inline cudaError_t launch_mix_cls(const MixArgs& a, int ncomp, cudaStream_t s) {
+    if constexpr (mix_two(OP, ROWS)) {
+        if (a.pl.cls == MIX_TWO) return launch_mix_t<T, OP, ROWS, MIX_TWO>(a, ncomp, s);
+    }
+    if (a.pl.cls != MIX_MULTI) return cudaErrorInvalidValue;
+    return launch_mix_t<T, OP, ROWS, MIX_MULTI>(a, ncomp, s);
+}
+
 template <typename T, int OP>
 inline cudaError_t launch_mix_op(bool rows, const MixArgs& a, int ncomp, cudaStream_t s) {
-    return rows ? launch_mix_t<T, OP, true>(a, ncomp, s) : launch_mix_t<T, OP, false>(a, ncomp, s);
+    return rows ? launch_mix_cls<T, OP, true>(a, ncomp, s) : launch_mix_cls<T, OP, false>(a, ncomp, s);
 }
 
 // instantiations, one unit per precision and group of operations

@@ -647,16 +647,16 @@ int Solver::mix_op(const PassArgs& A, bool f64, bool in_f64, bool out_f64) const
     const uintptr_t ain = dry ? 0 : (uintptr_t)A.in, aout = dry ? 0 : (uintptr_t)A.out;
     const uintptr_t cb = f64 ? 16 : 8;
     if (ain % (rin ? (in_f64 ? 8 : 4) : cb) != 0 || aout % (rout ? (out_f64 ? 8 : 4) : cb) != 0) return -1;
-    return M > 0 && mix_plan_of(M, op, f64) ? op : -1;
+    return M > 0 && mix_plan_of(M, op, A.axis == 0, f64) ? op : -1;
 }
 
 // the factorisation of a length, searched once per solver; nullptr: none
-const MixPlan* Solver::mix_plan_of(int M, int op, bool f64) const {
-    const std::array<int, 3> key{M, op, f64 ? 1 : 0};
+const MixPlan* Solver::mix_plan_of(int M, int op, bool rows, bool f64) const {
+    const std::array<int, 4> key{M, op, rows ? 1 : 0, f64 ? 1 : 0};
     auto it = mix_plans.find(key);
     if (it == mix_plans.end()) {
         MixPlan p{};
-        if (!mix_plan(M, op, f64 ? 1 : 0, p) || !mix_fits(p, op, f64 ? 1 : 0)) p.ns = 0;
+        if (!mix_plan(M, op, rows, f64 ? 1 : 0, p) || !mix_fits(p, op, f64 ? 1 : 0)) p.ns = 0;
         it = mix_plans.emplace(key, p).first;
     }
     return it->second.ns ? &it->second : nullptr;
@@ -714,7 +714,7 @@ void Solver::mix_args(const PassArgs& A, int op, bool f64, bool in_f64, bool out
         m.ax_b = b;
         m.ax_l = A.axis;
     }
-    m.pl = *mix_plan_of(mix_length(A.st[0]), op, f64);
+    m.pl = *mix_plan_of(mix_length(A.st[0]), op, A.axis == 0, f64);
     // the tile depends on the extents only: searched once per solver
     const std::array<int, 7> key{m.pl.M, op, f64 ? 1 : 0, A.axis == 0 ? 1 : 0, A.n_a, A.n_b, A.ncomp};
     auto it = mix_tiles.find(key);
@@ -727,8 +727,8 @@ void Solver::mix_args(const PassArgs& A, int op, bool f64, bool in_f64, bool out
 }
 
 const void* Solver::mix_table(const MixPlan& p, bool f64) {
-    int64_t key = ((int64_t)1 << 50) + ((int64_t)p.M << 20) + (f64 ? 1 : 0);
-    for (int s = 0; s < p.ns; ++s) key += (int64_t)(p.st[s].R - 1) << (4 + 4 * s);
+    int64_t key = ((int64_t)1 << 50) + ((int64_t)p.M << 24) + (f64 ? 1 : 0);
+    for (int s = 0; s < p.ns; ++s) key += (int64_t)(p.st[s].R - 1) << (1 + 5 * s);
     auto it = twiddles.find(key);
     if (it != twiddles.end()) return it->second;
     std::vector<double> w(2 * (size_t)std::max(p.ntw, 1), 0.0);
