@@ -314,10 +314,9 @@ struct GStage {
 // Fused passes visit the outer index in mirror pairs (0, 1, M-1, 2, M-2, ...,
 // M/2) when the Green's function is folded along it, so the folded Green slab
 // read for o is read again for M-o while it is still in L2.
+// (odd extents end with the pair (M-1)/2, (M+1)/2; every index comes once)
 __device__ __forceinline__ int mirror_order(int by, int nouter, int fold) {
-    if (fold != nouter || fold < 4) return by;
-    if (by == 0) return 0;
-    if (by == nouter - 1) return nouter / 2;
+    if (fold != nouter || by == 0) return by;
     const int m = (by + 1) >> 1;
     return (by & 1) ? m : nouter - m;
 }

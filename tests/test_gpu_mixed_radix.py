@@ -122,6 +122,23 @@ def test_mixed_radix_rot_matches_oracle(nglob, odiff):
         assert rel_l2(got, ref) <= tol
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,tol", [(64, 1e-12), (32, 2e-6)])
+@pytest.mark.parametrize("lda,type_", [(1, 0), (3, 1)])
+def test_odd_folded_outer_extent_of_a_register_fused_pass(precision, tol, lda, type_):
+    """64-point fused y columns whose outer direction (z, periodic, 25 points)
+    is folded: the order in mirror pairs visits every plane once."""
+    nglob = [16, 32, 25]
+    h, L = _lengths(nglob, CELL_CENTER)
+    bc = _bc("PPUUPP", lda)
+    rhs = _rhs(nglob, lda, "PPUUPP", CELL_CENTER)
+    ref = oracle_solve(nglob, lda, bc, h, L, CELL_CENTER, HEJ_2, rhs, type_=type_, odiff=1 if type_ else 0)
+    _, s = make_solver(nglob, lda, bc, h, L, CELL_CENTER, HEJ_2, odiff=1 if type_ else 0, precision=precision)
+    fused = [p for p in s.plan_json(type_)["passes"] if p["fused"]]
+    assert [(p["axis"], p["fast"]) for p in fused] == [(1, 1)]
+    assert rel_l2(from_user(_solve(s, to_user(rhs), type_), lda, nglob), ref) <= tol
+
+
 def _kinds(nglob, bc, center, precision=32):
     t = pf.Topology(0, 1, list(nglob))
     h, L = _lengths(nglob, center)
