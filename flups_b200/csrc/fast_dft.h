@@ -18,6 +18,7 @@ struct Prefetch {
 };
 
 struct ColArgs {
+    int chain;              // launched behind the solve's previous pass (launch_pass)
     const void* in;
     void* out;
     int nx;                 // columns along x (complex elements)
@@ -61,6 +62,7 @@ enum { COL_TILE_DEFAULT = 0, COL_TILE_256 = 1, COL_TILE_128 = 2 };
 // each row, Green's multiply (STD) or curl and Green's multiply (ROT, three
 // components), inverse DFT, in place.
 struct RowFusedArgs {
+    int chain;                   // as in ColArgs
     const void* in;
     void* out;
     int n1, n2;                  // rows (i1, i2), i1 < n1 fastest
@@ -82,6 +84,7 @@ struct RowFusedArgs {
 };
 
 struct RowArgs {
+    int chain;              // as in ColArgs
     const void* in;
     void* out;
     int nrows;              // rows per component

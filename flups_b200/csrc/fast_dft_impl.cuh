@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(TX * (L / R1), (Occ<TX * (L / R1), MODE == 2, 
     const C* tws = stage_twiddles<F>(a.tws, sm + TX * F::SC);
     T* gs = reinterpret_cast<T*>(sm + TX * F::SC + F::TW_SMEM);
     if constexpr (MODE == 2) stage_green<T, L, TX>(a, gs, o);
+    pass_begin();
     // lanes outside the array read its first element and drop it (no branch)
     const C* in = valid ? reinterpret_cast<const C*>(a.in) + comp * a.in_cstr + (int64_t)o * a.in_ostr + x + (int64_t)p * a.in_lstr
                         : reinterpret_cast<const C*>(a.in);
@@ -542,6 +543,7 @@ __global__ void __launch_bounds__(3 * TX * (L / R1), FLB_ROT_MINB) col_rot_kerne
     const C* tws = stage_twiddles<F>(a.tws, sm + 3 * TX * F::SC);
     T* gs = reinterpret_cast<T*>(sm + 3 * TX * F::SC + F::TW_SMEM);
     stage_green<T, L, TX>(a, gs, o);
+    pass_begin();
     // lanes outside the array read its first element and drop it (no branch)
     const C* in = valid ? reinterpret_cast<const C*>(a.in) + comp * a.in_cstr + (int64_t)o * a.in_ostr + x + (int64_t)p * a.in_lstr
                         : reinterpret_cast<const C*>(a.in);
@@ -673,6 +675,7 @@ __global__ void __launch_bounds__(WARPS * 32, RowFusedOcc<T>::blocks) row_fused_
         for (int e = p; e < CH; e += P) cp_async<16>(gs + e * PER, g + e * PER);
         cp_async_commit();
     }
+    pass_begin();
     const C* in = reinterpret_cast<const C*>(a.in) + comp * a.cstr + (int64_t)i1 * a.s1 + (int64_t)i2 * a.s2 + p;
     C v[R1];
 #pragma unroll
@@ -764,6 +767,7 @@ __global__ void __launch_bounds__(NT * 96, RowFusedOcc<T>::per_sm / (NT * 96) > 
         for (int e = p; e < CH; e += P) cp_async<16>(gs + e * PER, gr + e * PER);
         cp_async_commit();
     }
+    pass_begin();
     const C* in = reinterpret_cast<const C*>(a.in) + comp * a.cstr + (int64_t)i1 * a.s1 + (int64_t)i2 * a.s2 + p;
     C v[R1];
 #pragma unroll
@@ -868,8 +872,7 @@ inline cudaError_t launch_row_rot_t(const RowFusedArgs& a, int ncomp, cudaStream
     if (cudaError_t e = smem_attr_once(attr, row_rot_kernel<T, L, R1, NT, SH>, smem); e != cudaSuccess) return e;
     const int64_t rows = (int64_t)a.n1 * a.n2;
     dim3 grid((unsigned)((rows + NT * LPW - 1) / (NT * LPW)), ncomp / 3);
-    row_rot_kernel<T, L, R1, NT, SH><<<grid, NT * 96, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pass(row_rot_kernel<T, L, R1, NT, SH>, grid, dim3(NT * 96), smem, s, a, a.chain);
 }
 
 // lines of first radix R1 whose P = L / R1 threads fit in one warp
@@ -892,8 +895,7 @@ inline cudaError_t launch_row_fused_t(const RowFusedArgs& a, int ncomp, cudaStre
     if (cudaError_t e = smem_attr_once(attr, row_fused_kernel<T, L, R1, WARPS, SH>, smem); e != cudaSuccess) return e;
     const int64_t rows = (int64_t)a.n1 * a.n2;
     dim3 grid((unsigned)((rows + WARPS * LPW - 1) / (WARPS * LPW)), ncomp);
-    row_fused_kernel<T, L, R1, WARPS, SH><<<grid, WARPS * 32, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pass(row_fused_kernel<T, L, R1, WARPS, SH>, grid, dim3(WARPS * 32), smem, s, a, a.chain);
 }
 
 template <typename T, int SH, bool ROT>
@@ -966,6 +968,7 @@ __global__ void __launch_bounds__(TX * (L / R1), ColRealOcc<T, R1, C2R, TX * (L 
     const int comp = blockIdx.z;
     const bool valid = x < a.nx;
     const C* tws = stage_twiddles<F>(a.tws, sm + TX * F::SC);
+    pass_begin();
     C v[R1];
     if constexpr (!C2R) {
         constexpr int NLD = (SH == SH_HALF) ? R1 / 2 : R1;
@@ -1071,6 +1074,7 @@ __global__ void __launch_bounds__(TXP * (L / R1), ColRealOcc<T, R1, C2R, TXP * (
     const int comp = blockIdx.z;
     const bool valid = x < a.nx, two = x + 1 < a.nx;
     const C* tws = stage_twiddles<F>(a.tws, sm + TXP * F::SC);
+    pass_begin();
     C* line = sm + c * F::SC;
     C v[R1];
     const T z = (T)0;
@@ -1197,6 +1201,7 @@ __global__ void __launch_bounds__(TR * (LH / R1), (Occ<TR * (LH / R1), false, Ro
     const bool valid = row < a.nrows;
     const int i1 = valid ? row % a.n1 : 0, i2 = valid ? row / a.n1 : 0;
     prefetch_ahead<true>(a.pf, TR, a.n1);
+    pass_begin();
     // rows past the end read the array's first elements and drop them (no branch)
     const IT* src = valid ? reinterpret_cast<const IT*>(a.in) + comp * a.in_cstr + (int64_t)i1 * a.in_s1 + (int64_t)i2 * a.in_s2 + 2 * p
                           : reinterpret_cast<const IT*>(a.in);
@@ -1275,6 +1280,7 @@ __global__ void __launch_bounds__(TR * (M / R1), (Occ<TR * (M / R1)>::blocks)) r
     const IT* src = reinterpret_cast<const IT*>(a.in) + comp * a.in_cstr + (int64_t)i1 * a.in_s1 + (int64_t)i2 * a.in_s2;
     C* line = sm + rr * F::SC;
     const C* tws = stage_twiddles<F>(a.tws, sm + TR * F::SC);
+    pass_begin();
     const C* tw = reinterpret_cast<const C*>(a.tw2);
     const int n = a.n, kind = a.kind, nsrc = a.nin;
     const T z = (T)0;
@@ -1460,6 +1466,7 @@ __global__ void __launch_bounds__(TR * (LH / R1), DctOcc<T, R1, TR * (LH / R1)>:
         w4 = w4s;
     }
     cp_async_commit();
+    pass_begin();
     const bool dst = (a.kind == LK_DST1 || a.kind == LK_DST2 || a.kind == LK_DST3 || a.kind == LK_DST4);
     // DCT-III rows of all N inputs: pre-processed from registers and lane
     // shuffles instead of a staged copy of the row
@@ -1733,6 +1740,7 @@ __global__ void __launch_bounds__(TR * (LH / R1), (Occ<TR * (LH / R1), false, Ro
         stage_table_part<C, LH>(a.tw, wsm);
         cp_async_commit();
     }
+    pass_begin();
     const C* src = reinterpret_cast<const C*>(a.in) + comp * a.in_cstr + (int64_t)i1 * a.in_s1 + (int64_t)i2 * a.in_s2;
     // stage the half spectrum X[0..LH] (line positions 0..LH-1, X[LH] kept aside in registers);
     // rows past the end read the array's first element and drop it (no branch)
@@ -1813,8 +1821,7 @@ inline cudaError_t launch_col_t(const ColArgs& a, int ncomp, cudaStream_t s) {
     static std::atomic<unsigned long long> attr{0};
     if (cudaError_t e = smem_attr_once(attr, col_dft_kernel<T, L, R1, TX, MODE, SH>, smem); e != cudaSuccess) return e;
     dim3 grid((a.nx + TX - 1) / TX, a.nouter, ncomp);
-    col_dft_kernel<T, L, R1, TX, MODE, SH><<<grid, TX * F::P, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pass(col_dft_kernel<T, L, R1, TX, MODE, SH>, grid, dim3(TX * F::P), smem, s, a, a.chain);
 }
 
 // CTA tiles of a column pass: THREADS threads = TX columns x P threads per
@@ -1874,8 +1881,7 @@ inline cudaError_t launch_rot_t(const ColArgs& a, int ncomp, cudaStream_t s) {
         static std::atomic<unsigned long long> attr{0};
         if (cudaError_t e = smem_attr_once(attr, col_rot_kernel<T, L, RT::R1, RT::TX, SH>, smem); e != cudaSuccess) return e;
         dim3 grid((a.nx + RT::TX - 1) / RT::TX, a.nouter, ncomp / 3);
-        col_rot_kernel<T, L, RT::R1, RT::TX, SH><<<grid, RT::THREADS, smem, s>>>(a);
-        return cudaGetLastError();
+        return launch_pass(col_rot_kernel<T, L, RT::R1, RT::TX, SH>, grid, dim3(RT::THREADS), smem, s, a, a.chain);
     }
 }
 
@@ -1918,15 +1924,13 @@ inline cudaError_t launch_colreal_t(const ColArgs& a, int ncomp, cudaStream_t s)
         static std::atomic<unsigned long long> attr{0};
         if (cudaError_t e = smem_attr_once(attr, col_real_pair_kernel<T, RT, L, R1, TXP, C2R, SH>, smem); e != cudaSuccess) return e;
         dim3 grid(((a.nx + 1) / 2 + TXP - 1) / TXP, a.nouter, ncomp);
-        col_real_pair_kernel<T, RT, L, R1, TXP, C2R, SH><<<grid, TXP * F::P, smem, s>>>(a);
-        return cudaGetLastError();
+        return launch_pass(col_real_pair_kernel<T, RT, L, R1, TXP, C2R, SH>, grid, dim3(TXP * F::P), smem, s, a, a.chain);
     }
     const size_t smem = (size_t)(TX * F::SC + F::TW_SMEM) * sizeof(typename CT<T>::C);
     static std::atomic<unsigned long long> attr{0};
     if (cudaError_t e = smem_attr_once(attr, col_real_kernel<T, RT, L, R1, TX, C2R, SH>, smem); e != cudaSuccess) return e;
     dim3 grid((a.nx + TX - 1) / TX, a.nouter, ncomp);
-    col_real_kernel<T, RT, L, R1, TX, C2R, SH><<<grid, TX * F::P, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pass(col_real_kernel<T, RT, L, R1, TX, C2R, SH>, grid, dim3(TX * F::P), smem, s, a, a.chain);
 }
 
 template <typename T, typename RT, bool C2R, int SH>
@@ -1973,8 +1977,7 @@ inline cudaError_t launch_r2r_t(const RowArgs& a, int ncomp, cudaStream_t s) {
     static std::atomic<unsigned long long> attr{0};
     if (cudaError_t e = smem_attr_once(attr, row_r2r_kernel<T, IT, OT, M, R1, TR>, smem); e != cudaSuccess) return e;
     dim3 grid((a.nrows + TR - 1) / TR, ncomp);
-    row_r2r_kernel<T, IT, OT, M, R1, TR><<<grid, TR * F::P, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pass(row_r2r_kernel<T, IT, OT, M, R1, TR>, grid, dim3(TR * F::P), smem, s, a, a.chain);
 }
 
 template <typename T, typename IT, typename OT>
@@ -2004,8 +2007,7 @@ inline cudaError_t launch_dct_t(const RowArgs& a, int ncomp, cudaStream_t s) {
     static std::atomic<unsigned long long> attr{0};
     if (cudaError_t e = smem_attr_once(attr, row_dct_kernel<T, IT, OT, LH, R1, TR, FAM>, smem); e != cudaSuccess) return e;
     dim3 grid((a.nrows + TR - 1) / TR, ncomp);
-    row_dct_kernel<T, IT, OT, LH, R1, TR, FAM><<<grid, TR * F::P, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pass(row_dct_kernel<T, IT, OT, LH, R1, TR, FAM>, grid, dim3(TR * F::P), smem, s, a, a.chain);
 }
 
 // n: the (even) transform length; LH = n / 2
@@ -2047,9 +2049,8 @@ inline cudaError_t launch_row_t(const RowArgs& a, int ncomp, cudaStream_t s) {
     else e = smem_attr_once(attr, row_r2c_kernel<T, XT, LH, R1, TR, HALF>, smem);
     if (e != cudaSuccess) return e;
     dim3 grid((a.nrows + TR - 1) / TR, ncomp);
-    if constexpr (C2R) row_c2r_kernel<T, XT, LH, R1, TR, HALF><<<grid, TR * F::P, smem, s>>>(a);
-    else row_r2c_kernel<T, XT, LH, R1, TR, HALF><<<grid, TR * F::P, smem, s>>>(a);
-    return cudaGetLastError();
+    if constexpr (C2R) return launch_pass(row_c2r_kernel<T, XT, LH, R1, TR, HALF>, grid, dim3(TR * F::P), smem, s, a, a.chain);
+    else return launch_pass(row_r2c_kernel<T, XT, LH, R1, TR, HALF>, grid, dim3(TR * F::P), smem, s, a, a.chain);
 }
 
 template <typename T, typename XT, bool C2R, bool HALF>

@@ -230,6 +230,7 @@ struct Solver {
     const flb::MixPlan* mix_plan_of(int M, int op, bool rows, bool f64) const;
     mutable std::map<std::array<int, 4>, flb::MixPlan> mix_plans;         // per length, operation, rows and precision
     mutable std::map<std::array<int, 7>, std::array<int, 2>> mix_tiles;   // and per extents: lines, threads per line
+    bool chain_passes = false;            // passes may be launched behind each other programmatically (solve)
     bool use_mix = true;                  // false while the no-allocation solve plans its passes
     // arguments of a fast launch, all but the twiddle tables; mode of a column pass
     void fast_args(const flb::PassArgs& A, int kind, bool in_f64, bool out_f64, flb::ColArgs& c, flb::RowArgs& r, int& mode) const;

@@ -259,8 +259,15 @@ __device__ __forceinline__ T load_elem(const void* p, int64_t off, int f64, int 
 }
 
 // ---------------------------------------------------------------- kernel
+struct LinePassArgs {
+    PassArgs A;
+    int in_f64, out_f64;
+};
+
 template <typename T>
-__global__ void __launch_bounds__(256) line_pass_kernel(const PassArgs A, int in_f64, int out_f64) {
+__global__ void __launch_bounds__(256) line_pass_kernel(const __grid_constant__ LinePassArgs P) {
+    const PassArgs& A = P.A;
+    const int in_f64 = P.in_f64, out_f64 = P.out_f64;
     using C = typename CT<T>::C;
     extern __shared__ __align__(16) unsigned char sm[];
     const int fused = A.fused;
@@ -274,6 +281,7 @@ __global__ void __launch_bounds__(256) line_pass_kernel(const PassArgs A, int in
     axes_of(A.axis, ax_a, ax_b);
     const int64_t total_slots = A.comps_together ? (int64_t)A.nlines * ncg : (int64_t)A.nlines * A.ncomp;
     const int64_t slot0 = (int64_t)blockIdx.x * S;
+    pass_begin();
 
     auto slot_pos = [&](int s, bool& valid) {
         SlotPos p;
@@ -469,8 +477,7 @@ cudaError_t launch_line_pass_t(const PassArgs& A, int in_f64, int out_f64, cudaS
     else nblocks = ((int64_t)A.nlines * A.ncomp + A.lines_per_cta - 1) / A.lines_per_cta;
     (void)ncg;
     if (nblocks <= 0) return cudaSuccess;
-    line_pass_kernel<T><<<(unsigned)nblocks, 256, smem, stream>>>(A, in_f64, out_f64);
-    return cudaGetLastError();
+    return launch_pass(line_pass_kernel<T>, dim3((unsigned)nblocks), dim3(256), smem, stream, LinePassArgs{A, in_f64, out_f64}, A.chain);
 }
 
 cudaError_t launch_line_pass(const PassArgs& A, int compute_f64, int in_f64, int out_f64, cudaStream_t stream) {

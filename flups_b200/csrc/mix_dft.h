@@ -80,6 +80,7 @@ struct MixPlan {
 };
 
 struct MixArgs {
+    int chain;                             // launched behind the solve's previous pass (launch_pass)
     const void* in;
     void* out;
     MixPlan pl;

@@ -245,6 +245,7 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
                              (int)(ROWS ? blockDim.x : blockDim.y), a.pl, reinterpret_cast<const C*>(a.tw)};
     const int M = a.pl.M, ns = a.pl.ns;
     const MixPos<PAIR, ROWS> W(a, c, TX, OP == MX_FUSED);
+    pass_begin();
     const auto& ok = W.ok;
     const int isl = (int)a.in_sl, osl = (int)a.out_sl;
     const C zero = mkc((T)0, (T)0);
@@ -503,6 +504,7 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
     const MixLine<T, ROWS, CLS> L{reinterpret_cast<C*>(smraw) + (ROWS ? c * a.pl.len : c), TX, (int)(ROWS ? threadIdx.x : threadIdx.y),
                              (int)(ROWS ? blockDim.x : blockDim.y), a.pl, reinterpret_cast<const C*>(a.tw)};
     const MixPos<PAIR, ROWS> W(a, c, TX, GREEN);
+    pass_begin();
     constexpr int H = MixPos<PAIR, ROWS>::H;
     const int M = a.pl.M, ns = a.pl.ns, R_last = a.pl.st[ns - 1].R, nq = a.pl.st[ns - 1].Q;
     const int isl = (int)a.in_sl, osl = (int)a.out_sl;
@@ -881,6 +883,7 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
                               (int)(ROWS ? blockDim.x : blockDim.y), a.pl, reinterpret_cast<const C*>(a.tw)};
     auto line = [&](int g) { return MixLine<T, ROWS, CLS>{L0.sm + g * plane, L0.es, L0.p, L0.P, L0.pl, L0.tw}; };
     const MixPos<false, ROWS> W(a, c, TX, true);
+    pass_begin();
     const int ns = a.pl.ns, nq = a.pl.st[ns - 1].Q;
     const int isl = (int)a.in_sl, osl = (int)a.out_sl;
     const C zero = mkc((T)0, (T)0);
@@ -989,9 +992,8 @@ inline cudaError_t launch_mix_t(const MixArgs& a, int ncomp, cudaStream_t s) {
     const size_t smem = (size_t)a.tx * a.pl.len * mix_planes(OP) * sizeof(typename CT<T>::C);
     if (a.tx < 1 || a.P < 1 || a.tx * a.P > MixOcc<T, CLS>::threads || smem > 227 * 1024) return cudaErrorInvalidValue;
     const unsigned gx = (unsigned)((units + a.tx - 1) / a.tx);
-    if constexpr (ROWS) kernel<<<dim3(gx, 1, ncomp), dim3(a.P, a.tx), smem, s>>>(a);
-    else kernel<<<dim3(gx, a.nb, ncomp), dim3(a.tx, a.P), smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pass(kernel, ROWS ? dim3(gx, 1, ncomp) : dim3(gx, a.nb, ncomp), ROWS ? dim3(a.P, a.tx) : dim3(a.tx, a.P), smem, s, a,
+                       a.chain);
 }
 
 template <typename T, int OP, bool ROWS>

@@ -90,6 +90,7 @@ struct PassArgs {
     int lines_per_cta;
     int fused;                   // 0: one stage; 1: stage0 -> multiply -> stage1
     int comps_together;          // ROT: the three components of a position in one CTA
+    int chain;                   // directly behind the same solve's previous pass on one stream
     LineStage st[2];
     MultSpec mult;
     int nlines;                  // number of line positions (n_a * n_b)

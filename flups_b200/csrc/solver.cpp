@@ -1008,6 +1008,7 @@ void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, boo
         MixArgs m;
         const int op = mix_op(A, f64, in_f64, out_f64);
         mix_args(A, op, f64, in_f64, out_f64, m);
+        m.chain = A.chain;
         m.tw = mix_table(m.pl, f64);
         if (mix_mirrors(op) && op >= MX_T2 && op != MX_FUSED_R) m.tw4 = twiddle(2 * m.N[0], f64);
         if (op == MX_T4 || op == MX_FUSED_44) {
@@ -1020,6 +1021,7 @@ void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, boo
     if (kind == 5) {
         RowFusedArgs f;
         rowfused_args(A, f);
+        f.chain = A.chain;
         f.tws = stage_table(L, f64, A.mult.mode == 2 ? fast_radix1_rowrot(L, f64 ? 1 : 0) : fast_radix1_rowfused(L, f64 ? 1 : 0));
         if (prefetch && A.mult.mode == 2) rowrot_prefetch(f, f64, L, A.ncomp);
         check_cuda(launch_fast_rowfused(f64 ? 1 : 0, A.mult.mode == 2, L, f, A.ncomp, stream), "fused row launch");
@@ -1029,6 +1031,7 @@ void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, boo
     RowArgs r;
     int mode = 0;
     fast_args(A, kind, in_f64, out_f64, c, r, mode);
+    c.chain = r.chain = A.chain;
     if (kind == 4) {
         r.tw2 = twiddle(L, f64);
         if (fast_dct_family(r.kind, r.n, L)) {
@@ -1221,6 +1224,7 @@ void Solver::run_pass(const PassArgs& Ain, bool f64, bool in_f64, bool out_f64, 
     double bytes = (double)A.n_src * A.nlines * nc * (A.st[0].in_cplx ? 2 : 1) * (in_f64 ? 8.0 : 4.0) +
                    (double)last.n_store * A.nlines * nc * (last.out_cplx ? 2 : 1) * (out_f64 ? 8.0 : 4.0);
     if (A.fused) bytes += (double)gfold_n[0] * gfold_n[1] * gfold_n[2] * es;
+    A.chain = chain_passes && pass_idx > 0 && !timing;
     const int k = timed_begin(name, bytes);
     if (fk) launch_fast(A, fk, f64, in_f64, out_f64);
     else check_cuda(launch_line_pass(A, f64 ? 1 : 0, in_f64 ? 1 : 0, out_f64 ? 1 : 0, stream), "line pass launch");
@@ -1835,8 +1839,12 @@ void Solver::solve(double* field, double* rhs, int type, int nbatch) {
     } else {
         const bool xl = xlast_ok(type);
         if (xl) swap_order();
+        // the passes behind each other on one stream, nothing between them
+        // (captured solves keep plain launches: graph edges are short already)
+        chain_passes = !capturing;
         do_fft_forward(din, nbatch);
         do_fft_backward_fused(dout, type, nbatch);
+        chain_passes = false;
         if (xl) swap_order();
     }
     collect_timing();
