@@ -128,15 +128,16 @@ void mix_twiddle_exponent(const MixPlan& p, int e, int* q, int* n) {
 }
 
 // lines per CTA and threads per line: the tile of the least cost, a product of
-//  - butterfly slots offered over those needed, whole warps counted,
-//  - the column tile's run of x: 128 bytes 1, 64 bytes 1.15, 32 bytes 1.35
-//    (400-point fused columns at 200^3, FP32: 156 us with 16 columns, 170 with
-//    8; FP64: 302 with 8, 354 with 4),
-//  - small against large CTAs: 128 to 160 threads ran best (several resident
-//    CTAs overlap one's barriers with another's loads; 240 points FP32: 41 us
-//    with 128 threads, 46 with 256),
-//  - too few resident threads (shared memory, registers), and too few CTAs for
-//    the 148 SMs.
+//  - butterfly slots offered over those needed, whole warps counted, and a
+//    CTA's fixed work,
+//  - the column tile's lanes past the last line and its run of x: 128 bytes 1,
+//    64 bytes 1.15, 32 bytes 1.35 (400-point fused columns at 200^3, FP32: 156
+//    us with 16 columns, 170 with 8; FP64: 302 with 8, 354 with 4),
+//  - resident threads: a CTA's warps go round the four schedulers, each with a
+//    quarter of the registers, so a fifth warp costs as much as four more (at
+//    200^3 FP32, real rows of 400 points: 8 x 16 threads 63 us, 10 x 16 77 us),
+//  - row tiles whose lanes straddle two lines in a bank group,
+//  - too few CTAs for the 148 SMs.
 void mix_tile(MixArgs& a, int f64, int op, bool rows, int64_t ncomp) {
     const size_t line = (size_t)a.pl.len * mix_planes(op) * (f64 ? 16 : 8);
     const int64_t lines = (int64_t)mix_units(a.na, mix_pairs(op), rows) * (rows ? a.nb : 1);
@@ -145,7 +146,7 @@ void mix_tile(MixArgs& a, int f64, int op, bool rows, int64_t ncomp) {
     int maxp = 1;
     for (int s = 0; s < a.pl.ns; ++s) maxp = std::max(maxp, a.pl.M / a.pl.st[s].R);
     // registers per thread of the kernel, and the resident threads per SM that hide its latencies
-    const int regs = a.pl.cls == MIX_TWO ? (f64 ? 168 : 128) : (f64 ? 128 : 80), want = f64 ? 384 : 480;
+    const int regs = a.pl.cls == MIX_TWO ? (f64 ? 168 : 128) : (f64 ? 128 : 80), want = 65536 / regs / 128 * 128;
     double best = 1e30;
     a.tx = 1;
     a.P = std::min(maxp, 32);
@@ -163,11 +164,16 @@ void mix_tile(MixArgs& a, int f64, int op, bool rows, int64_t ncomp) {
         if (!rows) {
             const int run = tx * (f64 ? 16 : 8);
             c *= run >= 128 ? 1.0 : (run >= 96 ? 1.03 : (run >= 64 ? 1.15 : (run >= 32 ? 1.35 : 1.8)));
+        } else if (P % (f64 ? 8 : 16) != 0) {
+            c *= 1.12;  // a bank group of lanes straddles two lines
         }
-        const int ctas_sm = std::min((int)(227 * 1024 / (smem + 1024)), 65536 / (regs * ((th + 31) / 32 * 32)));
+        // a CTA's warps go round the four schedulers, each with a quarter of the registers
+        const int quarter = (th + 127) / 128;
+        const int ctas_sm = std::min((int)(227 * 1024 / (smem + 1024)), 16384 / (regs * 32 * quarter));
         const int resident = std::max(1, ctas_sm) * th;
         if (resident < want) c *= 1.0 + 0.5 * ((double)want / resident - 1.0);
         const double ctas = (double)((lines + tx - 1) / tx) * outer;
+        if (!rows) c *= (double)((lines + tx - 1) / tx) * tx / lines;  // lanes past the last column
         if (ctas < 148) c *= 1.3 * 148 / ctas;
         else if (ctas < 296) c *= 1.0 + 0.3 * (296 - ctas) / 148;
         if (c < best) {

@@ -40,13 +40,13 @@ constexpr int kMixStages = 4;
 // kernel classes: two to four stages of smaller radices, or two of larger ones
 enum MixClass : int { MIX_MULTI = 0, MIX_TWO = 1 };
 constexpr int mix_threads(int f64, int cls) { return cls == MIX_TWO && f64 ? 128 : 256; }
-// the operations compiled in class TWO: column passes (row passes lose by it:
-// 288-point real rows of a 145 x 121 x 101 grid, FP32, 20 us in 9 x 8 x 4, 26
-// us in 18 x 16; their lanes already run along the line, so fewer threads
-// share it)
-constexpr bool mix_two(int op, bool rows) {
-    return !rows && (op == MX_R2C || op == MX_C2R || op == MX_C2C_F || op == MX_C2C_I || op == MX_FUSED);
-}
+// the operations compiled in class TWO: column passes of the complex kinds and
+// r2c / c2r.  Row passes lose by it (288-point real rows of a 145 x 121 x 101
+// grid, FP32, 20 us in three stages, 26 in two: few threads share a line there),
+// and so do the r2r and fused real ones, whose last stage holds two butterflies
+// and their twiddles (180-point fused z of a 250 x 150 x 180 box, FP64, 60 ->
+// 92 us).
+constexpr bool mix_two(int op, bool rows) { return !rows && op <= MX_FUSED; }
 // radices of a class.  small: of a last stage that takes two or three
 // butterflies in one thread.  The limits are those that keep the butterflies
 // in the class's registers.
