@@ -77,7 +77,7 @@ int flups_get_pass_stats(struct Solver* s, int maxn, double* ms_total, double* b
 int flups_b200_plan_json(struct Solver* s, int type, int nbatch, char* out, int len);
 
 /* Use (1, default) or bypass (0) the register-resident power-of-two DFT
- * kernels; with 0 every pass runs through the general line-pass kernel.
+ * kernels and the mixed-radix ones; with 0 every pass runs through the general line-pass kernel.
  * For cross-checking the two kernel families. */
 void flups_b200_set_fast_kernels(struct Solver* s, int on);
 
