@@ -1839,9 +1839,14 @@ void Solver::solve(double* field, double* rhs, int type, int nbatch) {
     } else {
         const bool xl = xlast_ok(type);
         if (xl) swap_order();
-        // the passes behind each other on one stream, nothing between them
-        // (captured solves keep plain launches: graph edges are short already)
-        chain_passes = !capturing;
+        // the passes behind each other on one stream, nothing between them;
+        // captured solves, the caller's own captures too, keep plain launches
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (!capturing && cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
+            cudaGetLastError();  // the legacy stream while another one captures: the launches report it
+            cap = cudaStreamCaptureStatusActive;
+        }
+        chain_passes = !capturing && cap == cudaStreamCaptureStatusNone;
         do_fft_forward(din, nbatch);
         do_fft_backward_fused(dout, type, nbatch);
         chain_passes = false;
