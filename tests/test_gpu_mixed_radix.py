@@ -123,6 +123,31 @@ def test_mixed_radix_rot_matches_oracle(nglob, odiff):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [20, 32])
+def test_solve_captured_by_the_caller_equals_the_plain_one(n):
+    """Back-to-back solves (passes launched behind each other) and the same
+    solve captured in a graph of the caller's own give the same bits."""
+    import torch
+    h, L = _lengths([n] * 3, CELL_CENTER)
+    _, s = make_solver([n] * 3, 1, _bc("UUUUUU"), h, L, CELL_CENTER, HEJ_2)
+    rhs = torch.from_numpy(to_user(_rhs([n] * 3, 1, "UUUUUU", CELL_CENTER))).cuda()
+    st = torch.cuda.Stream()
+    s.set_stream(st)
+    s.set_async(True)
+    plain, out = torch.zeros_like(rhs), torch.zeros_like(rhs)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        s.solve(plain, rhs)
+    st.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        s.solve(out, rhs)
+    g.replay()
+    torch.cuda.synchronize()
+    assert s.last_error() == 0 and torch.equal(out, plain)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("precision,tol", [(64, 1e-12), (32, 2e-6)])
 @pytest.mark.parametrize("lda,type_", [(1, 0), (3, 1)])
 def test_odd_folded_outer_extent_of_a_register_fused_pass(precision, tol, lda, type_):
