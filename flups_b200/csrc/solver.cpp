@@ -337,18 +337,7 @@ const void* Solver::twiddle(int M, bool f64) {
         w[2 * q] = (double)cosl(a);
         w[2 * q + 1] = (double)sinl(a);
     }
-    void* d = nullptr;
-    if (f64) {
-        check_cuda(cudaMalloc(&d, w.size() * sizeof(double)), "twiddle allocation");
-        check_cuda(cudaMemcpy(d, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice), "twiddle upload");
-    } else {
-        std::vector<float> wf(w.size());
-        for (size_t i = 0; i < w.size(); ++i) wf[i] = (float)w[i];
-        check_cuda(cudaMalloc(&d, wf.size() * sizeof(float)), "twiddle allocation");
-        check_cuda(cudaMemcpy(d, wf.data(), wf.size() * sizeof(float), cudaMemcpyHostToDevice), "twiddle upload");
-    }
-    twiddles[key] = d;
-    return d;
+    return twiddles[key] = upload_table(w, f64);
 }
 
 // ---------------------------------------------------------------- stages
@@ -756,18 +745,19 @@ const void* Solver::type4_table(int N, bool f64) {
     return twiddles[key] = upload_table(w, f64);
 }
 
-// device copy of a table of complex values, in the working precision
+// Device copy of a table of complex values, in the working precision.  Copied
+// on the solver's stream and waited for: a plain cudaMemcpy from pageable
+// memory may return before the data has arrived, and a non-blocking stream is
+// not ordered behind it.
 void* Solver::upload_table(const std::vector<double>& w, bool f64) {
+    std::vector<float> wf;
+    if (!f64) wf.assign(w.begin(), w.end());
+    const void* src = f64 ? (const void*)w.data() : (const void*)wf.data();
+    const size_t bytes = w.size() * (f64 ? sizeof(double) : sizeof(float));
     void* d = nullptr;
-    if (f64) {
-        check_cuda(cudaMalloc(&d, w.size() * sizeof(double)), "twiddle allocation");
-        check_cuda(cudaMemcpy(d, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice), "twiddle upload");
-    } else {
-        std::vector<float> wf(w.size());
-        for (size_t i = 0; i < w.size(); ++i) wf[i] = (float)w[i];
-        check_cuda(cudaMalloc(&d, wf.size() * sizeof(float)), "twiddle allocation");
-        check_cuda(cudaMemcpy(d, wf.data(), wf.size() * sizeof(float), cudaMemcpyHostToDevice), "twiddle upload");
-    }
+    check_cuda(cudaMalloc(&d, bytes), "twiddle allocation");
+    check_cuda(cudaMemcpyAsync(d, src, bytes, cudaMemcpyHostToDevice, stream), "twiddle upload");
+    check_cuda(cudaStreamSynchronize(stream), "twiddle upload");
     return d;
 }
 
@@ -1142,18 +1132,7 @@ const void* Solver::stage_table(int n, bool f64, int r1) {
         w[2 * e] = (double)cosl(a);
         w[2 * e + 1] = (double)sinl(a);
     }
-    void* d = nullptr;
-    if (f64) {
-        check_cuda(cudaMalloc(&d, w.size() * sizeof(double)), "twiddle allocation");
-        check_cuda(cudaMemcpy(d, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice), "twiddle upload");
-    } else {
-        std::vector<float> wf(w.size());
-        for (size_t i = 0; i < w.size(); ++i) wf[i] = (float)w[i];
-        check_cuda(cudaMalloc(&d, wf.size() * sizeof(float)), "twiddle allocation");
-        check_cuda(cudaMemcpy(d, wf.data(), wf.size() * sizeof(float), cudaMemcpyHostToDevice), "twiddle upload");
-    }
-    twiddles[key] = d;
-    return d;
+    return twiddles[key] = upload_table(w, f64);
 }
 
 const void* Solver::twiddle_plain(int L, bool f64) {
@@ -1166,18 +1145,7 @@ const void* Solver::twiddle_plain(int L, bool f64) {
         w[2 * q] = (double)cosl(a);
         w[2 * q + 1] = (double)sinl(a);
     }
-    void* d = nullptr;
-    if (f64) {
-        check_cuda(cudaMalloc(&d, w.size() * sizeof(double)), "twiddle allocation");
-        check_cuda(cudaMemcpy(d, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice), "twiddle upload");
-    } else {
-        std::vector<float> wf(w.size());
-        for (size_t i = 0; i < w.size(); ++i) wf[i] = (float)w[i];
-        check_cuda(cudaMalloc(&d, wf.size() * sizeof(float)), "twiddle allocation");
-        check_cuda(cudaMemcpy(d, wf.data(), wf.size() * sizeof(float), cudaMemcpyHostToDevice), "twiddle upload");
-    }
-    twiddles[key] = d;
-    return d;
+    return twiddles[key] = upload_table(w, f64);
 }
 
 // Restrict a pass to the slab [slab_lo, slab_hi) of dimension slab_dim (not
@@ -1392,12 +1360,12 @@ void Solver::compute_green() {
     }
     if (!table.empty() && !dry) {
         check_cuda(cudaMalloc(&d_table, table.size() * sizeof(double)), "LGF table");
-        check_cuda(cudaMemcpy(d_table, table.data(), table.size() * sizeof(double), cudaMemcpyHostToDevice), "LGF table");
+        check_cuda(cudaMemcpyAsync(d_table, table.data(), table.size() * sizeof(double), cudaMemcpyHostToDevice, stream), "LGF table");
         E.table = d_table;
     }
     if (!far.empty() && !dry) {
         check_cuda(cudaMalloc(&d_far, far.size() * sizeof(FarTerm)), "far field");
-        check_cuda(cudaMemcpy(d_far, far.data(), far.size() * sizeof(FarTerm), cudaMemcpyHostToDevice), "far field");
+        check_cuda(cudaMemcpyAsync(d_far, far.data(), far.size() * sizeof(FarTerm), cudaMemcpyHostToDevice, stream), "far field");
         E.far = d_far;
         E.nfar = (int)far.size();
         E.far_log = far_log;
