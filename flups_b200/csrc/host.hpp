@@ -234,7 +234,8 @@ struct Solver {
     bool use_mix = true;                  // false while the no-allocation solve plans its passes
     // arguments of a fast launch, all but the twiddle tables; mode of a column pass
     void fast_args(const flb::PassArgs& A, int kind, bool in_f64, bool out_f64, flb::ColArgs& c, flb::RowArgs& r, int& mode) const;
-    void launch_fast(const flb::PassArgs& A, int kind, bool f64, bool in_f64, bool out_f64);
+    void launch_fast(const flb::PassArgs& A, int kind, bool f64, bool in_f64, bool out_f64, bool go);
+    void make_tables();
     void rowfused_args(const flb::PassArgs& A, flb::RowFusedArgs& f) const;
     void ensure_buffers(int nbatch);
     flb::LineStage stage_forward(const flb::DirPlan& p, int ip, bool f64);

@@ -992,7 +992,8 @@ void Solver::rowfused_args(const PassArgs& A, RowFusedArgs& f) const {
     }
 }
 
-void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, bool out_f64) {
+// go = false: make the tables of the pass without launching it
+void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, bool out_f64, bool go) {
     const int L = A.st[0].M;
     if (kind == 6) {
         MixArgs m;
@@ -1005,6 +1006,7 @@ void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, boo
             m.tw4 = twiddle(2 * m.N[0], f64);
             m.tw8 = type4_table(m.N[0], f64);
         }
+        if (!go) return;
         check_cuda(launch_mix(f64 ? 1 : 0, op, A.axis == 0, m, A.ncomp, stream), "mixed-radix pass launch");
         return;
     }
@@ -1013,6 +1015,7 @@ void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, boo
         rowfused_args(A, f);
         f.chain = A.chain;
         f.tws = stage_table(L, f64, A.mult.mode == 2 ? fast_radix1_rowrot(L, f64 ? 1 : 0) : fast_radix1_rowfused(L, f64 ? 1 : 0));
+        if (!go) return;
         if (prefetch && A.mult.mode == 2) rowrot_prefetch(f, f64, L, A.ncomp);
         check_cuda(launch_fast_rowfused(f64 ? 1 : 0, A.mult.mode == 2, L, f, A.ncomp, stream), "fused row launch");
         return;
@@ -1031,16 +1034,19 @@ void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, boo
         } else {
             r.tws = stage_table(L, f64);
         }
+        if (!go) return;
         check_cuda(launch_fast_r2r(f64, L, r, A.ncomp, stream), "r2r row launch");
         return;
     }
     if (kind == 3) {
         c.tws = stage_table(L, f64, fast_radix1_colreal(L, f64 ? 1 : 0));
+        if (!go) return;
         check_cuda(launch_fast_colreal(f64, A.st[0].spec[0].kind == LK_C2R, L, c, A.ncomp, stream), "column r2c/c2r launch");
         return;
     }
     if (kind == 1) {
         c.tws = stage_table(L, f64, fast_radix1_mode(L, f64 ? 1 : 0, mode));
+        if (!go) return;
         if (force_tile) {
             c.tile = force_tile;
         } else if (!tuned_tile.empty()) {
@@ -1060,6 +1066,7 @@ void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, boo
     }
     r.tw = twiddle_plain(L, f64);
     r.tws = stage_table(L / 2, f64, fast_radix1_row(L / 2, f64 ? 1 : 0));
+    if (!go) return;
     const bool c2r = A.st[0].spec[0].kind == LK_C2R;
     if (prefetch) row_prefetch(r, f64, c2r, L, A.ncomp);
     check_cuda(launch_fast_row(f64, c2r, L, r, A.ncomp, stream), "row DFT launch");
@@ -1194,7 +1201,7 @@ void Solver::run_pass(const PassArgs& Ain, bool f64, bool in_f64, bool out_f64, 
     if (A.fused) bytes += (double)gfold_n[0] * gfold_n[1] * gfold_n[2] * es;
     A.chain = chain_passes && pass_idx > 0 && !timing;
     const int k = timed_begin(name, bytes);
-    if (fk) launch_fast(A, fk, f64, in_f64, out_f64);
+    if (fk) launch_fast(A, fk, f64, in_f64, out_f64, true);
     else check_cuda(launch_line_pass(A, f64 ? 1 : 0, in_f64 ? 1 : 0, out_f64 ? 1 : 0, stream), "line pass launch");
     timed_end(k);
 }
@@ -1513,7 +1520,43 @@ void Solver::setup() {
     build_ksym();
     plan_xlast();
     ensure_buffers(1);
+    make_tables();
     is_setup = true;
+}
+
+// The twiddle tables of every pass of a solve of device arrays, made at
+// set-up: such a solve then allocates and uploads nothing, and its caller may
+// capture the first one in a graph (an allocation ends a capture).  Other pass
+// orders and the general pass with the fast kernels off make theirs when they
+// first run.
+void Solver::make_tables() {
+    const bool f64 = (precision == 64);
+    for (int type : {STD, ROT}) {
+        if (type == ROT && (lda != 3 || !have_diff)) continue;
+        const bool xl = xlast_ok(type);
+        if (xl) swap_order();
+        dry = true;
+        dry_passes.clear();
+        dry_flags.clear();
+        dry_names.clear();
+        dry_fast.clear();
+        do_fft_forward(nullptr, 1);
+        do_fft_backward_fused(nullptr, type, 1);
+        for (size_t i = 0; i < dry_passes.size(); ++i) {
+            const PassArgs& A = dry_passes[i];
+            if (dry_fast[i]) {
+                launch_fast(A, dry_fast[i], f64, dry_flags[i] & 2, dry_flags[i] & 4, false);
+            } else {
+                for (int s2 = 0; s2 <= A.fused; ++s2) twiddle(A.st[s2].M, f64);
+            }
+        }
+        dry_passes.clear();
+        dry_flags.clear();
+        dry_names.clear();
+        dry_fast.clear();
+        dry = false;
+        if (xl) swap_order();
+    }
 }
 
 // The curl symbols K_{d,c}(i) of a solver that can run ROT (three components
