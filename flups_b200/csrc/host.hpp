@@ -264,6 +264,8 @@ struct Solver {
     void* ksym = nullptr;
     int kstr = 0;
     void build_ksym();
+    void* ksym64 = nullptr;               // FP64 symbols of an FP32 solver's mixed-radix ROT pass
+    const void* ksym_f64();
     // x-last order of an all-unbounded 3-D problem: z (r2c), y, x, so that the
     // last direction (forward DFT, multiply, inverse DFT) runs along
     // contiguous rows, one warp per row.  Solves of device arrays use it; the

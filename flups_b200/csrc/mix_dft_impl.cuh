@@ -870,8 +870,11 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
 // one CTA, one after the other through the stages, together in the last one,
 // where a thread holds the same wave numbers of all three and forms
 //   u_g = G (w_{g+2} K_{g+1,g+2} - w_{g+1} K_{g+2,g+1})  (indices mod 3)
-// between the two transforms.  Along the line the symbols change with k;
-// those of the other two directions are constants of the thread.
+// between the two transforms, in FP64 with FP64 symbols whatever the working
+// precision (one rounding of the result, as in the general pass; the FP32 pass
+// at 200^3 takes 833 us for it, 662 with an FP32 curl, the general pass 4750).
+// Along the line the symbols change with k; those of the other two directions
+// are constants of the thread.
 template <typename T, bool ROWS, int CLS>
 __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::blocks) mix_rot_kernel(const __grid_constant__ MixArgs a) {
     using C = typename CT<T>::C;
@@ -909,15 +912,16 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
     {
         const T* g = W.template green<T>(a, 0);
         const int gl = (int)a.g_sl;
-        const C* K = reinterpret_cast<const C*>(a.ksym);
+        const double2* K = reinterpret_cast<const double2*>(a.ksym);
         // K_{d,c}: kc[d][0] for c = d + 1, kc[d][1] for c = d + 2 (mod 3)
-        C kc[3][2];
-        const C* kl[2];
+        double2 kc[3][2];
+        const double2* kl[2];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const int i = d == a.ax_a ? W.ia[0] : W.ib;
 #pragma unroll
-            for (int e = 0; e < 2; ++e) kc[d][e] = d == a.ax_l ? zero : __ldg(K + (3 * d + (d + 1 + e) % 3) * a.kstr + i);
+            for (int e = 0; e < 2; ++e)
+                kc[d][e] = d == a.ax_l ? make_double2(0.0, 0.0) : __ldg(K + (3 * d + (d + 1 + e) % 3) * a.kstr + i);
         }
 #pragma unroll
         for (int e = 0; e < 2; ++e) kl[e] = K + (3 * a.ax_l + (a.ax_l + 1 + e) % 3) * a.kstr;
@@ -936,15 +940,18 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
 #pragma unroll
                 for (int j = 0; j < R; ++j) {
                     const int k = q + nq * j;
-                    const T gv = __ldg(g + mix_fold(k, a.f_l) * gl);
-                    const C ka = __ldg(kl[0] + k), kb = __ldg(kl[1] + k);
+                    const double gv = (double)__ldg(g + mix_fold(k, a.f_l) * gl);
+                    const double2 ka = __ldg(kl[0] + k), kb = __ldg(kl[1] + k);
                     C u[3];
 #pragma unroll
                     for (int h = 0; h < 3; ++h) {
                         const int p = (h + 1) % 3, q2 = (h + 2) % 3;
-                        const C kp = p == a.ax_l ? ka : kc[p][0];    // K_{h+1, h+2}
-                        const C kq = q2 == a.ax_l ? kb : kc[q2][1];  // K_{h+2, h+1}
-                        u[h] = cscale(csub(cmul(v[q2][j], kp), cmul(v[p][j], kq)), gv);
+                        const double2 kp = p == a.ax_l ? ka : kc[p][0];    // K_{h+1, h+2}
+                        const double2 kq = q2 == a.ax_l ? kb : kc[q2][1];  // K_{h+2, h+1}
+                        const double2 wq = make_double2((double)v[q2][j].x, (double)v[q2][j].y);
+                        const double2 wp = make_double2((double)v[p][j].x, (double)v[p][j].y);
+                        const double2 r = csub(cmul(wq, kp), cmul(wp, kq));
+                        u[h] = mkc((T)(r.x * gv), (T)(r.y * gv));
                     }
 #pragma unroll
                     for (int h = 0; h < 3; ++h) v[h][j] = u[h];

@@ -281,6 +281,7 @@ Solver::~Solver() {
     if (xlast_active) swap_order();
     if (ksym) cudaFree(ksym);
     if (xksym) cudaFree(xksym);
+    if (ksym64) cudaFree(ksym64);
     if (h2d_stream) {
         for (int k = 0; k < kSlabs; ++k) {
             cudaEventDestroy(ev_in[k]);
@@ -697,7 +698,6 @@ void Solver::mix_args(const PassArgs& A, int op, bool f64, bool in_f64, bool out
         m.f_l = A.mult.gfold[A.axis];
     }
     if (op == MX_ROT) {
-        m.ksym = ksym;
         m.kstr = kstr;
         m.ax_a = a;
         m.ax_b = b;
@@ -1001,6 +1001,7 @@ void Solver::launch_fast(const PassArgs& A, int kind, bool f64, bool in_f64, boo
         mix_args(A, op, f64, in_f64, out_f64, m);
         m.chain = A.chain;
         m.tw = mix_table(m.pl, f64);
+        if (op == MX_ROT) m.ksym = ksym_f64();
         if (mix_mirrors(op) && op >= MX_T2 && op != MX_FUSED_R) m.tw4 = twiddle(2 * m.N[0], f64);
         if (op == MX_T4 || op == MX_FUSED_44) {
             m.tw4 = twiddle(2 * m.N[0], f64);
@@ -1584,6 +1585,21 @@ void Solver::build_ksym() {
     check_cuda(cudaStreamSynchronize(stream), "curl symbol tables");
 }
 
+// The reference order's curl symbols in FP64: the mixed-radix ROT pass forms
+// the curl in FP64 in either precision, as the general pass does.
+const void* Solver::ksym_f64() {
+    FLB_CHECK(!xlast_active, "the x-last order has no FP64 curl symbols");
+    if (precision == 64) return ksym;
+    if (!ksym64) {
+        int n[3];
+        for (int d = 0; d < 3; ++d) n[d] = st[ndim].n[d];
+        check_cuda(cudaMalloc(&ksym64, (size_t)9 * kstr * 2 * sizeof(double)), "curl symbol tables");
+        check_cuda(launch_ksym_table(mult_spec(ROT), n, kstr, ksym64, 1, stream), "curl symbol tables");
+        check_cuda(cudaStreamSynchronize(stream), "curl symbol tables");
+    }
+    return ksym64;
+}
+
 // A solver set up for a share keeps only its columns [own[2], own[3]) of the
 // folded Green's spectrum (x is not folded there), rows on 128-byte
 // boundaries; `green` is placed where the full array would start, so the
@@ -1648,6 +1664,7 @@ size_t Solver::device_bytes(int nbatch) const {
     total += (size_t)gstr[2] * gfold_n[2] * es;
     if (ksym) total += (size_t)9 * kstr * 2 * es;
     if (xksym) total += (size_t)9 * xkstr * 2 * es;
+    if (ksym64) total += (size_t)9 * kstr * 2 * sizeof(double);
     return total;
 }
 
