@@ -3,7 +3,8 @@
     python -m flups_b200.build          (or flups_b200.build.build())
 
 Steps: turn kernel/farfield.json into a C include of coefficient tables,
-then compile csrc/*.cu and csrc/*.cpp into flups_b200/libflups_b200.so.
+then compile csrc/*.cu and csrc/*.cpp into flups_b200/libflups_b200.so
+(mix_unit.cu once per mixed-radix operation, precision and direction).
 """
 import json
 import math
@@ -18,6 +19,7 @@ BUILD = PKG / "_build"
 LIB = PKG / "libflups_b200.so"
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+MIX_OPS = 15  # operations of the mixed-radix passes (MixOp, csrc/mix_dft.h)
 
 
 def gen_farfield():
@@ -44,20 +46,25 @@ def gen_farfield():
     return out
 
 
-def sources():
-    return sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cpp"))
+def units():
+    """(source, object name, defines) of every translation unit; the longest first."""
+    mix = [(CSRC / "mix_unit.cu", f"mix_op{op:02d}_{name}_{'rows' if rows else 'cols'}",
+            (f"-DFLB_MIX_OP={op}", f"-DFLB_MIX_T={real}", f"-DFLB_MIX_ROWS={str(rows).lower()}"))
+           for op in reversed(range(MIX_OPS)) for real, name in (("float", "f32"), ("double", "f64")) for rows in (False, True)]
+    rest = [s for s in sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cpp")) if s.name != "mix_unit.cu"]
+    return mix + [(s, s.stem, ()) for s in rest]
 
 
 def build(verbose=False, extra=()):
     gen_farfield()
     objs, jobs = [], []
-    for src in sources():
-        obj = BUILD / (src.stem + ".o")
+    for src, name, defines in units():
+        obj = BUILD / (name + ".o")
         deps = [src] + list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.hpp")) + \
             list((PKG.parent / "include").glob("*.h")) + [BUILD / "farfield_data.inc"]
         if not obj.exists() or any(d.stat().st_mtime > obj.stat().st_mtime for d in deps):
             cmd = [NVCC, *ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-I", str(BUILD),
-                   "-I", str(PKG.parent / "include"), "--expt-relaxed-constexpr", *extra]
+                   "-I", str(PKG.parent / "include"), "--expt-relaxed-constexpr", *defines, *extra]
             if src.suffix == ".cpp":
                 cmd += ["-x", "cu"]
             cmd += ["-c", str(src), "-o", str(obj)]

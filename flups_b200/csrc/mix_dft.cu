@@ -1,9 +1,9 @@
 // Mixed-radix line passes: factorisation, tiles and dispatch (kernels in
-// mix_dft_impl.cuh, instantiated in mix_*.cu so that the units compile in
-// parallel).
+// mix_dft_impl.cuh, one module per operation, precision and direction:
+// mix_unit.cu).
 #include <algorithm>
 
-#include "mix_dft_impl.cuh"
+#include "mix_dft.h"
 
 namespace flb {
 
@@ -196,24 +196,30 @@ void mix_tile(MixArgs& a, int f64, int op, bool rows, int64_t ncomp) {
 
 bool mix_fits(const MixPlan& p, int op, int f64) { return (size_t)p.len * mix_planes(op) * (f64 ? 16 : 8) <= 227 * 1024; }
 
+template <int OP>
+static cudaError_t launch_op(int f64, bool rows, const MixArgs& a, int ncomp, cudaStream_t s) {
+    if (f64) return rows ? launch_mix_op<double, OP, true>(a, ncomp, s) : launch_mix_op<double, OP, false>(a, ncomp, s);
+    return rows ? launch_mix_op<float, OP, true>(a, ncomp, s) : launch_mix_op<float, OP, false>(a, ncomp, s);
+}
+
 cudaError_t launch_mix(int f64, int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s) {
     switch (op) {
-        case MX_C2C_F:
-        case MX_C2C_I: return f64 ? launch_mix_c2c_f64(op, rows, a, ncomp, s) : launch_mix_c2c_f32(op, rows, a, ncomp, s);
-        case MX_R2C:
-        case MX_C2R: return f64 ? launch_mix_real_f64(op, rows, a, ncomp, s) : launch_mix_real_f32(op, rows, a, ncomp, s);
-        case MX_T1:
-        case MX_T2:
-        case MX_T3:
-        case MX_T4: return f64 ? launch_mix_r2r_f64(op, rows, a, ncomp, s) : launch_mix_r2r_f32(op, rows, a, ncomp, s);
-        case MX_FUSED_R:
-        case MX_FUSED_23:
-        case MX_FUSED_32:
-        case MX_FUSED_11:
-        case MX_FUSED_44:
-            return f64 ? launch_mix_fused_real_f64(op, rows, a, ncomp, s) : launch_mix_fused_real_f32(op, rows, a, ncomp, s);
-        case MX_ROT: return launch_mix_rot(f64, rows, a, ncomp, s);
-        case MX_FUSED: return launch_mix_fused(f64, rows, a, ncomp, s);
+        case MX_C2C_F: return launch_op<MX_C2C_F>(f64, rows, a, ncomp, s);
+        case MX_C2C_I: return launch_op<MX_C2C_I>(f64, rows, a, ncomp, s);
+        case MX_R2C: return launch_op<MX_R2C>(f64, rows, a, ncomp, s);
+        case MX_C2R: return launch_op<MX_C2R>(f64, rows, a, ncomp, s);
+        case MX_FUSED: return launch_op<MX_FUSED>(f64, rows, a, ncomp, s);
+        case MX_T2: return launch_op<MX_T2>(f64, rows, a, ncomp, s);
+        case MX_T3: return launch_op<MX_T3>(f64, rows, a, ncomp, s);
+        case MX_T1: return launch_op<MX_T1>(f64, rows, a, ncomp, s);
+        case MX_T4: return launch_op<MX_T4>(f64, rows, a, ncomp, s);
+        case MX_FUSED_R: return launch_op<MX_FUSED_R>(f64, rows, a, ncomp, s);
+        case MX_FUSED_23: return launch_op<MX_FUSED_23>(f64, rows, a, ncomp, s);
+        case MX_FUSED_32: return launch_op<MX_FUSED_32>(f64, rows, a, ncomp, s);
+        case MX_FUSED_11: return launch_op<MX_FUSED_11>(f64, rows, a, ncomp, s);
+        case MX_FUSED_44: return launch_op<MX_FUSED_44>(f64, rows, a, ncomp, s);
+        // one launch per field: the three components of a line position are the CTA's
+        case MX_ROT: return ncomp == 3 ? launch_op<MX_ROT>(f64, rows, a, 1, s) : cudaErrorInvalidValue;
     }
     return cudaErrorInvalidValue;
 }

@@ -36,6 +36,15 @@ constexpr bool mix_mirrors(int op) {
     return op == MX_R2C || op == MX_C2R || op == MX_T2 || op == MX_T3 || op == MX_FUSED_R || op == MX_FUSED_23 || op == MX_FUSED_32;
 }
 
+// lines or pairs of lines among na neighbouring positions (MixPos pairs them)
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int mix_units(int na, bool pair, bool rows) {
+    if (!pair) return na;
+    return rows ? (na + 1) / 2 : 8 * (na / 16) + (na % 16 < 8 ? na % 16 : 8);
+}
+
 constexpr int kMixStages = 4;
 // kernel classes: two to four stages of smaller radices, or two of larger ones
 enum MixClass : int { MIX_MULTI = 0, MIX_TWO = 1 };
@@ -117,6 +126,8 @@ void mix_twiddle_exponent(const MixPlan& p, int e, int* q, int* n);
 void mix_tile(MixArgs& a, int f64, int op, bool rows, int64_t ncomp);
 // rows: lines along the lanes' direction (x); ncomp: grid z
 cudaError_t launch_mix(int f64, int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
+// one operation in one precision and direction (mix_unit.cu)
+template <typename T, int OP, bool ROWS> cudaError_t launch_mix_op(const MixArgs& a, int ncomp, cudaStream_t s);
 // whether one line position of the pass fits in shared memory
 bool mix_fits(const MixPlan& p, int op, int f64);
 

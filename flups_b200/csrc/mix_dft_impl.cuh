@@ -196,10 +196,6 @@ struct MixLine {
 // 2i + 1, columns x and x + 8 of 16 (each half of a pair then loads whole
 // runs).  Lines outside the array point at position 0 and are neither loaded
 // nor stored.
-__host__ __device__ inline int mix_units(int na, bool pair, bool rows) {
-    if (!pair) return na;
-    return rows ? (na + 1) / 2 : 8 * (na / 16) + (na % 16 < 8 ? na % 16 : 8);
-}
 template <bool PAIR, bool ROWS>
 struct MixPos {
     static constexpr int H = PAIR ? 2 : 1;
@@ -1004,29 +1000,12 @@ inline cudaError_t launch_mix_t(const MixArgs& a, int ncomp, cudaStream_t s) {
 }
 
 template <typename T, int OP, bool ROWS>
-inline cudaError_t launch_mix_cls(const MixArgs& a, int ncomp, cudaStream_t s) {
+cudaError_t launch_mix_op(const MixArgs& a, int ncomp, cudaStream_t s) {
     if constexpr (mix_two(OP, ROWS)) {
         if (a.pl.cls == MIX_TWO) return launch_mix_t<T, OP, ROWS, MIX_TWO>(a, ncomp, s);
     }
     if (a.pl.cls != MIX_MULTI) return cudaErrorInvalidValue;
     return launch_mix_t<T, OP, ROWS, MIX_MULTI>(a, ncomp, s);
 }
-
-template <typename T, int OP>
-inline cudaError_t launch_mix_op(bool rows, const MixArgs& a, int ncomp, cudaStream_t s) {
-    return rows ? launch_mix_cls<T, OP, true>(a, ncomp, s) : launch_mix_cls<T, OP, false>(a, ncomp, s);
-}
-
-// instantiations, one unit per precision and group of operations
-cudaError_t launch_mix_c2c_f32(int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
-cudaError_t launch_mix_c2c_f64(int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
-cudaError_t launch_mix_real_f32(int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
-cudaError_t launch_mix_real_f64(int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
-cudaError_t launch_mix_r2r_f32(int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
-cudaError_t launch_mix_r2r_f64(int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
-cudaError_t launch_mix_fused_real_f32(int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
-cudaError_t launch_mix_fused_real_f64(int op, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
-cudaError_t launch_mix_rot(int f64, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
-cudaError_t launch_mix_fused(int f64, bool rows, const MixArgs& a, int ncomp, cudaStream_t s);
 
 }  // namespace flb

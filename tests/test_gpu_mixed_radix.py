@@ -205,3 +205,18 @@ def test_lengths_outside_the_radices_stay_on_the_general_pass():
         assert kinds == [6] * 5
         pf.load_library().flups_b200_set_fast_kernels(s._solver, 0)
         assert [p["fast"] for p in s.plan_json()["passes"] if p["name"] != "green"] == [0] * 5
+
+
+def test_one_module_per_mixed_radix_operation():
+    """A module is loaded whole at its first launch: each operation, precision
+    and direction is a translation unit of its own."""
+    import re
+    from flups_b200 import build
+    ops = re.findall(r"^    MX_\w+ = (\d+),", (build.CSRC / "mix_dft.h").read_text(), re.M)
+    assert sorted(map(int, ops)) == list(range(build.MIX_OPS))
+    units = [d for s, _, d in build.units() if s.name == "mix_unit.cu"]
+    assert len(units) == len(set(units)) == 4 * build.MIX_OPS
+    names = [n for _, n, _ in build.units()]
+    assert len(names) == len(set(names))
+    others = [s for s in build.CSRC.glob("*.cu") if s.name != "mix_unit.cu" and "mix_dft_impl.cuh" in s.read_text()]
+    assert not others
