@@ -218,5 +218,5 @@ def test_one_module_per_mixed_radix_operation():
     assert len(units) == len(set(units)) == 4 * build.MIX_OPS
     names = [n for _, n, _ in build.units()]
     assert len(names) == len(set(names))
-    others = [s for s in build.CSRC.glob("*.cu") if s.name != "mix_unit.cu" and "mix_dft_impl.cuh" in s.read_text()]
+    others = [s for s in build.CSRC.glob("*.cu") if s.name != "mix_unit.cu" and '#include "mix_dft_impl.cuh"' in s.read_text()]
     assert not others
