@@ -2484,7 +2484,6 @@ std::string Solver::plan_json(int type, int nbatch) {
     do_fft_forward(nullptr, nbatch);
     do_fft_backward_fused(nullptr, type, nbatch);
     if (xl) swap_order();
-    dry = false;
     for (size_t i = 0; i < dry_passes.size(); ++i) {
         const PassArgs& A = dry_passes[i];
         const int es = (dry_flags[i] & 1) ? 8 : 4;
@@ -2509,8 +2508,18 @@ std::string Solver::plan_json(int type, int nbatch) {
             }
             o += "]}";
         }
-        o += "]}";
+        o += "]";
+        if (dry_fast[i] == 6) {
+            const int op = mix_op(A, dry_flags[i] & 1, dry_flags[i] & 2, dry_flags[i] & 4);
+            const MixPlan& p = *mix_plan_of(mix_length(A.st[0]), op, A.axis == 0, dry_flags[i] & 1);
+            snprintf(b, sizeof(b), ",\"mix\":{\"op\":%d,\"two\":%d,\"radices\":[", op, p.cls == MIX_TWO ? 1 : 0);
+            o += b;
+            for (int k = 0; k < p.ns; ++k) o += (k ? "," : "") + std::to_string(p.st[k].R);
+            o += "]}";
+        }
+        o += "}";
     }
+    dry = false;
     o += "],\"xlast\":";
     o += xl ? "1" : "0";
     o += "}";
