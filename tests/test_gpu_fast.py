@@ -82,18 +82,18 @@ CASES = [
 @pytest.mark.parametrize("name,nglob,lda,bcv,center,kernel", CASES, ids=[c[0] for c in CASES])
 def test_fast_fp64_matches_oracle(name, nglob, lda, bcv, center, kernel):
     got, ref, plan = _run(nglob, lda, bcv, center, kernel, 64, True)
-    assert any(p["fast"] for p in plan["passes"] if p["name"] != "green"), "fast kernels not selected"
+    assert any(p["fast"] in (1, 2, 3, 4, 5) for p in plan["passes"] if p["name"] != "green"), "fast kernels not selected"
     assert rel_l2(got, ref) <= 1e-12
 
 
 @pytest.mark.parametrize("name,nglob", [(c[0], c[1]) for c in CASES if c[0].endswith("_r48")])
 def test_radix48_lines_run_the_register_dft(name, nglob):
-    """The 768-point lines of the radix-48 cases run the register DFT (not the
-    general line pass) in FP32, so the parity cases above check that path."""
+    """The 768-point lines of the radix-48 cases run the register DFT (not a
+    mixed-radix or general pass) in FP32, so the parity cases above check that path."""
     case = next(c for c in CASES if c[0] == name)
     _, _, plan = _run(case[1], case[2], case[3], case[4], case[5], 32, True)
     long_passes = [p for p in plan["passes"] if p["name"] != "green" and p["st"][0]["M"] == 768]
-    assert long_passes and all(p["fast"] for p in long_passes), long_passes
+    assert long_passes and all(p["fast"] in (1, 2, 3, 4, 5) for p in long_passes), long_passes
 
 
 @pytest.mark.parametrize("name,nglob,lda,bcv,center,kernel", CASES, ids=[c[0] for c in CASES])

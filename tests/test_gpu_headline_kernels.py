@@ -119,7 +119,7 @@ def _oracle(name, nglob, lda, bcv, center, kernel, rhs, type_=0, odiff=0):
 def _check_fast(plan, M, axis):
     sel = [p for p in plan["passes"] if p["name"] != "green" and p["axis"] == axis and p["st"][0]["M"] == M]
     assert sel, f"no pass of {M}-point lines along axis {axis}"
-    assert all(p["fast"] for p in sel), sel
+    assert all(p["fast"] in (1, 2, 3, 4, 5) for p in sel), sel
 
 
 @pytest.mark.parametrize("device", [False, True], ids=["host", "device"])

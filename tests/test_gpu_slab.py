@@ -96,18 +96,21 @@ def test_slab_refuses_other_problems():
         SlabRank(s, 0, 2)
 
 
-def test_slab_peers_refused_without_register_dft_y_passes():
-    """50^3 unbounded has 100-point lines, which the register DFTs do not
-    cover: the y passes run the general line pass, which cannot store into
-    the owners' column arrays, so connecting the peers is refused (-2) and
-    the all-to-all form still equals the one-rank solve."""
+@pytest.mark.parametrize("n,kind", [(50, 6), (34, 0)])
+def test_slab_peers_refused_without_register_dft_y_passes(n, kind):
+    """50^3 unbounded has 100-point lines, 34^3 68-point ones, which the
+    register DFTs do not cover: the y passes are mixed-radix (kind 6) or
+    general (0) ones, which cannot store into the owners' column arrays, so
+    connecting the peers is refused (-2) and the all-to-all form still equals
+    the one-rank solve."""
     import torch
     from flups_b200.slab import SlabRank, solve_local
-    n, world = 50, 2
+    world = 2
     rng = np.random.default_rng(5)
     rhs = torch.from_numpy(to_user(rng.standard_normal((1, n, n, n)))).cuda()
     t, s = make_solver([n] * 3, 1, UNB, [1.0 / n] * 3, [1.0] * 3, CELL_CENTER, HEJ_2, precision=64)
     s.set_xlast(False)  # the slab steps run the reference's pass order
+    assert all(p["fast"] == kind for p in s.plan_json()["passes"] if p["name"] != "green")
     ref = torch.zeros_like(rhs)
     s.solve(ref, rhs)
     torch.cuda.synchronize()

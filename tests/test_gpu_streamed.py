@@ -5,8 +5,8 @@ arithmetic as whole-array passes, so a solve with host arrays must equal the
 solve of the same data in device arrays in the same (reference) pass order
 bit for bit: one call, async calls
 back to back (each with its own input), a batch, an in-place call, a
-vector ROT solve, and grids that run the general line pass instead of the
-register DFTs."""
+vector ROT solve, and grids that run the mixed-radix passes or the general
+line pass instead of the register DFTs."""
 import numpy as np
 import pytest
 
@@ -20,7 +20,8 @@ CASES = [
     # (name, nglob, lda, bcv, center, kernel, precision)
     ("unb64_fast_fp64", [64] * 3, 1, UNB, CELL_CENTER, LGF_2, 64),
     ("unb64_fast_fp32", [64] * 3, 1, UNB, CELL_CENTER, HEJ_2, 32),
-    ("unb_ragged_general", [24, 20, 18], 1, UNB, CELL_CENTER, CHAT_2, 64),
+    ("unb_ragged_mixed_radix", [24, 20, 18], 1, UNB, CELL_CENTER, CHAT_2, 64),
+    ("unb_ragged_general", [34, 19, 17], 1, UNB, CELL_CENTER, CHAT_2, 64),
     ("mixed_bc_node", [17, 9, 9], 1, [[[0], [1]], [[3], [3]], [[4], [4]]], NODE_CENTER, CHAT_2, 64),
 ]
 
@@ -51,6 +52,9 @@ def _device_solve(s, u, type_=0, nbatch=1):
 def test_host_equals_device(name, nglob, lda, bcv, center, kernel, precision):
     import torch
     t, s = _setup(nglob, lda, bcv, center, kernel, precision)
+    kinds = {p["fast"] for p in s.plan_json()["passes"] if p["name"] != "green"}
+    if "mixed_radix" in name or "general" in name:
+        assert (6 if "mixed_radix" in name else 0) in kinds
     rng = np.random.default_rng(5)
     u = to_user(rng.standard_normal((lda,) + tuple(nglob)))
     ref = _device_solve(s, u)
