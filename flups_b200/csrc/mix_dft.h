@@ -112,9 +112,10 @@ struct MixArgs {
     const void* green;
     int64_t g_sa, g_sb, g_sl;
     int f_a, f_b, f_l;                     // fold lengths (0 = none)
-    // FP64 curl symbols K_{d,c}(i) at (3 d + c) kstr + i; the directions of a, b and the line
+    // FP64 curl symbols K_{d,c}(i) at (3 d + c) kstr + i, imaginary where bit 3 d + c of kim is set, else real;
+    // the directions of a, b and the line
     const void* ksym;
-    int kstr, ax_a, ax_b, ax_l;
+    int kstr, kim, ax_a, ax_b, ax_l;
 };
 
 // Factorisation of M for a pass of operation `op`; false when M has a prime

@@ -868,7 +868,8 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
 //   u_g = G (w_{g+2} K_{g+1,g+2} - w_{g+1} K_{g+2,g+1})  (indices mod 3)
 // between the two transforms, in FP64 with FP64 symbols whatever the working
 // precision (one rounding of the result, as in the general pass; the FP32 pass
-// at 200^3 takes 833 us for it, 662 with an FP32 curl, the general pass 4750).
+// at 200^3 takes 772 us for it, 663 with an FP32 curl, the general pass 4750:
+// 13 conversions between the precisions per wave number).
 // Along the line the symbols change with k; those of the other two directions
 // are constants of the thread.
 template <typename T, bool ROWS, int CLS>
@@ -909,15 +910,19 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
         const T* g = W.template green<T>(a, 0);
         const int gl = (int)a.g_sl;
         const double2* K = reinterpret_cast<const double2*>(a.ksym);
+        // a table K_{d,c} is real or imaginary throughout (kim): one value of each
+        auto symbol = [](const double2* p) {
+            const double2 z = __ldg(p);
+            return z.x + z.y;
+        };
         // K_{d,c}: kc[d][0] for c = d + 1, kc[d][1] for c = d + 2 (mod 3)
-        double2 kc[3][2];
+        double kc[3][2];
         const double2* kl[2];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const int i = d == a.ax_a ? W.ia[0] : W.ib;
 #pragma unroll
-            for (int e = 0; e < 2; ++e)
-                kc[d][e] = d == a.ax_l ? make_double2(0.0, 0.0) : __ldg(K + (3 * d + (d + 1 + e) % 3) * a.kstr + i);
+            for (int e = 0; e < 2; ++e) kc[d][e] = d == a.ax_l ? 0.0 : symbol(K + (3 * d + (d + 1 + e) % 3) * a.kstr + i);
         }
 #pragma unroll
         for (int e = 0; e < 2; ++e) kl[e] = K + (3 * a.ax_l + (a.ax_l + 1 + e) % 3) * a.kstr;
@@ -937,16 +942,16 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
                 for (int j = 0; j < R; ++j) {
                     const int k = q + nq * j;
                     const double gv = (double)__ldg(g + mix_fold(k, a.f_l) * gl);
-                    const double2 ka = __ldg(kl[0] + k), kb = __ldg(kl[1] + k);
+                    const double ka = symbol(kl[0] + k), kb = symbol(kl[1] + k);
                     C u[3];
 #pragma unroll
                     for (int h = 0; h < 3; ++h) {
                         const int p = (h + 1) % 3, q2 = (h + 2) % 3;
-                        const double2 kp = p == a.ax_l ? ka : kc[p][0];    // K_{h+1, h+2}
-                        const double2 kq = q2 == a.ax_l ? kb : kc[q2][1];  // K_{h+2, h+1}
-                        const double2 wq = make_double2((double)v[q2][j].x, (double)v[q2][j].y);
-                        const double2 wp = make_double2((double)v[p][j].x, (double)v[p][j].y);
-                        const double2 r = csub(cmul(wq, kp), cmul(wp, kq));
+                        const double kp = p == a.ax_l ? ka : kc[p][0];    // K_{h+1, h+2}
+                        const double kq = q2 == a.ax_l ? kb : kc[q2][1];  // K_{h+2, h+1}
+                        const C wq = (a.kim >> (3 * p + q2)) & 1 ? cmul_pi(v[q2][j]) : v[q2][j];
+                        const C wp = (a.kim >> (3 * q2 + p)) & 1 ? cmul_pi(v[p][j]) : v[p][j];
+                        const double2 r = make_double2((double)wq.x * kp - (double)wp.x * kq, (double)wq.y * kp - (double)wp.y * kq);
                         u[h] = mkc((T)(r.x * gv), (T)(r.y * gv));
                     }
 #pragma unroll

@@ -699,6 +699,8 @@ void Solver::mix_args(const PassArgs& A, int op, bool f64, bool in_f64, bool out
     }
     if (op == MX_ROT) {
         m.kstr = kstr;
+        for (int d = 0; d < 3; ++d)
+            for (int c = 0; c < 3; ++c) m.kim |= (A.mult.kfact[d][c][1] != 0.0) << (3 * d + c);
         m.ax_a = a;
         m.ax_b = b;
         m.ax_l = A.axis;
