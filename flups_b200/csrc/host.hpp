@@ -167,7 +167,7 @@ struct Solver {
     std::vector<int> dry_flags;
     std::vector<std::string> dry_names;
     std::vector<int> dry_fast;
-    bool use_fast = true;                 // register-resident power-of-two kernels where they apply
+    bool use_fast = true;                 // register-DFT and mixed-radix kernels where they apply
     // ---------------------------------------------------------------- per-pass timing
     bool timing = false;
     int pass_idx = 0;
@@ -231,7 +231,7 @@ struct Solver {
     mutable std::map<std::array<int, 4>, flb::MixPlan> mix_plans;         // per length, operation, rows and precision
     mutable std::map<std::array<int, 7>, std::array<int, 2>> mix_tiles;   // and per extents: lines, threads per line
     bool chain_passes = false;            // passes may be launched behind each other programmatically (solve)
-    bool use_mix = true;                  // false while the no-allocation solve plans its passes
+    bool use_mix = true;                  // false in the Green's set-up and while the no-allocation solve plans its passes
     // arguments of a fast launch, all but the twiddle tables; mode of a column pass
     void fast_args(const flb::PassArgs& A, int kind, bool in_f64, bool out_f64, flb::ColArgs& c, flb::RowArgs& r, int& mode) const;
     void launch_fast(const flb::PassArgs& A, int kind, bool f64, bool in_f64, bool out_f64, bool go);

@@ -1,6 +1,8 @@
 #pragma once
 // Mixed-radix line passes: lengths 2^a 3^b 5^c 7^d 11^e 13^f in two to four
-// stages, for every line the register DFTs (fast_dft_impl.cuh) do not take.
+// stages of radices up to 16 (13 in FP64), or, for complex columns that would
+// take three, in two of radices up to 32 (20 in FP64), for the lines the
+// register DFTs (fast_dft_impl.cuh) do not take.
 //
 // A line sits in shared memory once.  A forward transform decimates in
 // frequency: stage s reads the R values of a butterfly, transforms them in

@@ -1,8 +1,9 @@
-// Butterflies of the mixed-radix line passes (mix_dft_impl.cuh): every radix
-// from 2 to 16 but 14, forward or inverse, on complex values in registers.
-// Primes by their symmetric sums (sum and difference of x_j and x_{R-j}, one
-// real product per pair), composites of coprime factors by the prime-factor
-// index maps (no twiddles between the two), 9 as 3 x 3; 2, 3, 4, 8 and 16 are
+// Butterflies of the mixed-radix line passes (mix_dft_impl.cuh): radices 2 to
+// 16, 18, 20, 24, 25 and 32, forward or inverse, on complex values in registers
+// (which of them a kernel class uses: mix_radix_ok).  Primes by their symmetric
+// sums (sum and difference of x_j and x_{R-j}, one real product per pair),
+// composites of coprime factors by the prime-factor index maps (no twiddles
+// between the two), 9 and 25 as squares of 3 and 5; 2, 3, 4, 8, 16 and 32 are
 // the register DFTs' own (cplx.cuh).
 #pragma once
 #include "cplx.cuh"

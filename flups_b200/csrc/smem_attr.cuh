@@ -26,12 +26,13 @@ inline cudaError_t smem_attr_once(std::atomic<unsigned long long>& devs, K kerne
 // with chain = 1 is launched when the last block of the pass before it ends,
 // instead of after that pass's memory has been flushed and its end reported:
 // its blocks set up (addresses, twiddles, Green's values: data no pass writes)
-// and wait in pass_begin() until every write of that pass is visible.  Five
-// passes, four gaps (FP32 free space, per solve): 64^3 28.7 -> 20.6 us, 128^3
-// 72.1 -> 61.7, 512^3 3540 -> 3483.  Letting the next pass start earlier
-// (griddepcontrol.launch_dependents at a pass's start) puts its waiting blocks
-// where the last wave has left room and not where they would run best: 512^3
-// 3756 us, a 1500 x 700 plane 53 us against 41.
+// and wait in pass_begin() until every write of that pass is visible.  2 to 3
+// us per gap saved (plain, chained; FP32 free space, HEJ_2, four gaps per solve, and
+// the FP64 1500 x 700 plane, two gaps): 64^3 28.7, 20.5 us; 128^3 72.7, 61.5;
+// plane 44.4, 39.0; 512^3 3600, 3590, within the scatter of its runs.  Letting
+// the next pass start earlier (griddepcontrol.launch_dependents at a pass's
+// start) puts its waiting blocks where the last wave has left room and not
+// where they would run best: 22.6, 63.5, 46.6 and 3794 us.
 __device__ __forceinline__ void pass_begin() {
 #if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
     asm volatile("griddepcontrol.wait;" ::: "memory");

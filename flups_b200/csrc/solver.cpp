@@ -1869,8 +1869,10 @@ void Solver::solve(double* field, double* rhs, int type, int nbatch) {
     } else {
         const bool xl = xlast_ok(type);
         if (xl) swap_order();
-        // the passes behind each other on one stream, nothing between them;
-        // captured solves, the caller's own captures too, keep plain launches
+        // the passes behind each other on one stream, nothing between them.
+        // Captured solves, the caller's own captures too, keep plain launches:
+        // the edges of a replayed graph cost no more than chained launches (64^3
+        // FP32 20.5 us either way, 128^3 62.4 against 61.5)
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (!capturing && cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
             cudaGetLastError();  // the legacy stream while another one captures: the launches report it
