@@ -870,11 +870,13 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
 //   u_g = G (w_{g+2} K_{g+1,g+2} - w_{g+1} K_{g+2,g+1})  (indices mod 3)
 // between the two transforms, in FP64 with FP64 symbols whatever the working
 // precision (one rounding of the result, as in the general pass; the FP32 pass
-// at 200^3 takes 772 us for it, 663 with an FP32 curl, the general pass 4750:
-// 13 conversions between the precisions per wave number).
+// at 200^3 takes 721 us for it, 663 with an FP32 curl, the general pass 4750:
+// 13 conversions between the precisions per wave number).  IMAG: every symbol
+// is imaginary (no walls), so the factor i is taken out (FP32 772 us without
+// that, FP64 1188 against 1315).
 // Along the line the symbols change with k; those of the other two directions
 // are constants of the thread.
-template <typename T, bool ROWS, int CLS>
+template <typename T, bool ROWS, int CLS, bool IMAG>
 __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::blocks) mix_rot_kernel(const __grid_constant__ MixArgs a) {
     using C = typename CT<T>::C;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -951,9 +953,13 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
                         const int p = (h + 1) % 3, q2 = (h + 2) % 3;
                         const double kp = p == a.ax_l ? ka : kc[p][0];    // K_{h+1, h+2}
                         const double kq = q2 == a.ax_l ? kb : kc[q2][1];  // K_{h+2, h+1}
-                        const C wq = (a.kim >> (3 * p + q2)) & 1 ? cmul_pi(v[q2][j]) : v[q2][j];
-                        const C wp = (a.kim >> (3 * q2 + p)) & 1 ? cmul_pi(v[p][j]) : v[p][j];
-                        const double2 r = make_double2((double)wq.x * kp - (double)wp.x * kq, (double)wq.y * kp - (double)wp.y * kq);
+                        C wq = v[q2][j], wp = v[p][j];
+                        if constexpr (!IMAG) {
+                            if ((a.kim >> (3 * p + q2)) & 1) wq = cmul_pi(wq);
+                            if ((a.kim >> (3 * q2 + p)) & 1) wp = cmul_pi(wp);
+                        }
+                        double2 r = make_double2((double)wq.x * kp - (double)wp.x * kq, (double)wq.y * kp - (double)wp.y * kq);
+                        if constexpr (IMAG) r = cmul_pi(r);
                         u[h] = mkc((T)(r.x * gv), (T)(r.y * gv));
                     }
 #pragma unroll
@@ -988,22 +994,30 @@ __global__ void __launch_bounds__(MixOcc<T, CLS>::threads, MixOcc<T, CLS>::block
     }
 }
 
-template <typename T, int OP, bool ROWS, int CLS>
-inline cudaError_t launch_mix_t(const MixArgs& a, int ncomp, cudaStream_t s) {
-    constexpr bool PAIR = mix_pairs(OP);
-    constexpr auto kernel = [] {
-        if constexpr (OP == MX_ROT) return mix_rot_kernel<T, ROWS, CLS>;
-        else if constexpr (OP >= MX_T2) return mix_real_kernel<T, OP, ROWS, CLS>;
-        else return mix_kernel<T, OP, ROWS, CLS>;
-    }();
-    static std::atomic<unsigned long long> attr{0};
+template <typename T, int OP, bool ROWS, int CLS, typename K>
+inline cudaError_t launch_mix_kernel(K kernel, std::atomic<unsigned long long>& attr, const MixArgs& a, int ncomp, cudaStream_t s) {
     if (cudaError_t e = smem_attr_once(attr, kernel, 227 * 1024); e != cudaSuccess) return e;
-    const int64_t units = (int64_t)mix_units(a.na, PAIR, ROWS) * (ROWS ? a.nb : 1);
+    const int64_t units = (int64_t)mix_units(a.na, mix_pairs(OP), ROWS) * (ROWS ? a.nb : 1);
     const size_t smem = (size_t)a.tx * a.pl.len * mix_planes(OP) * sizeof(typename CT<T>::C);
     if (a.tx < 1 || a.P < 1 || a.tx * a.P > MixOcc<T, CLS>::threads || smem > 227 * 1024) return cudaErrorInvalidValue;
     const unsigned gx = (unsigned)((units + a.tx - 1) / a.tx);
     return launch_pass(kernel, ROWS ? dim3(gx, 1, ncomp) : dim3(gx, a.nb, ncomp), ROWS ? dim3(a.P, a.tx) : dim3(a.tx, a.P), smem, s, a,
                        a.chain);
+}
+
+template <typename T, int OP, bool ROWS, int CLS>
+inline cudaError_t launch_mix_t(const MixArgs& a, int ncomp, cudaStream_t s) {
+    static std::atomic<unsigned long long> attr{0};
+    if constexpr (OP == MX_ROT) {
+        static std::atomic<unsigned long long> attr_im{0};
+        // the six tables of the curl (d != c) all imaginary: no walls
+        if ((a.kim & 0b011101110) == 0b011101110) return launch_mix_kernel<T, OP, ROWS, CLS>(mix_rot_kernel<T, ROWS, CLS, true>, attr_im, a, ncomp, s);
+        return launch_mix_kernel<T, OP, ROWS, CLS>(mix_rot_kernel<T, ROWS, CLS, false>, attr, a, ncomp, s);
+    } else if constexpr (OP >= MX_T2) {
+        return launch_mix_kernel<T, OP, ROWS, CLS>(mix_real_kernel<T, OP, ROWS, CLS>, attr, a, ncomp, s);
+    } else {
+        return launch_mix_kernel<T, OP, ROWS, CLS>(mix_kernel<T, OP, ROWS, CLS>, attr, a, ncomp, s);
+    }
 }
 
 template <typename T, int OP, bool ROWS>
