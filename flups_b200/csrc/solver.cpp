@@ -326,18 +326,21 @@ size_t Solver::alloc_size() const {
     return std::max(m, topo_phys->memsize());
 }
 
+// W_n^q = exp(-2 pi i q / n), rounded once.  pi in long double: that of a
+// double turns entries near a full turn by 2.4e-16, more than their rounding.
+static void root_of_unity(int64_t q, int64_t n, double* w) {
+    const long double a = -6.283185307179586476925286766559005768L * (long double)q / (long double)n;
+    w[0] = (double)cosl(a);
+    w[1] = (double)sinl(a);
+}
+
 const void* Solver::twiddle(int M, bool f64) {
     const int64_t key = (int64_t)M * 2 + (f64 ? 1 : 0);
     auto it = twiddles.find(key);
     if (it != twiddles.end()) return it->second;
-    // W_{2M}^q = exp(-2 pi i q / (2M)), q in [0, 2M), evaluated in FP64
+    // W_{2M}^q, q in [0, 2M)
     std::vector<double> w(4 * (size_t)M);
-    for (int q = 0; q < 2 * M; ++q) {
-        // reduce to the first quadrant for accuracy: angle = -pi q / M
-        const long double a = -(long double)M_PI * (long double)q / (long double)M;
-        w[2 * q] = (double)cosl(a);
-        w[2 * q + 1] = (double)sinl(a);
-    }
+    for (int q = 0; q < 2 * M; ++q) root_of_unity(q, 2 * (int64_t)M, &w[2 * q]);
     return twiddles[key] = upload_table(w, f64);
 }
 
@@ -726,9 +729,7 @@ const void* Solver::mix_table(const MixPlan& p, bool f64) {
     for (int e = 0; e < p.ntw; ++e) {
         int q = 0, n = 1;
         mix_twiddle_exponent(p, e, &q, &n);
-        const long double a = -2.0L * (long double)M_PI * (long double)q / (long double)n;
-        w[2 * e] = (double)cosl(a);
-        w[2 * e + 1] = (double)sinl(a);
+        root_of_unity(q, n, &w[2 * e]);
     }
     return twiddles[key] = upload_table(w, f64);
 }
@@ -739,11 +740,7 @@ const void* Solver::type4_table(int N, bool f64) {
     auto it = twiddles.find(key);
     if (it != twiddles.end()) return it->second;
     std::vector<double> w(2 * (size_t)(N / 2));
-    for (int j = 0; j < N / 2; ++j) {
-        const long double a = -2.0L * (long double)M_PI * (long double)(4 * j + 1) / (8.0L * (long double)N);
-        w[2 * j] = (double)cosl(a);
-        w[2 * j + 1] = (double)sinl(a);
-    }
+    for (int j = 0; j < N / 2; ++j) root_of_unity(4 * j + 1, 8 * (int64_t)N, &w[2 * j]);
     return twiddles[key] = upload_table(w, f64);
 }
 
@@ -1138,9 +1135,7 @@ const void* Solver::stage_table(int n, bool f64, int r1) {
     for (int e = 0; e < len; ++e) {
         int q = 0, M = 1;
         fast_stage_exponent(n, r1, e, &q, &M);
-        const long double a = -2.0L * (long double)M_PI * (long double)q / (long double)M;
-        w[2 * e] = (double)cosl(a);
-        w[2 * e + 1] = (double)sinl(a);
+        root_of_unity(q, M, &w[2 * e]);
     }
     return twiddles[key] = upload_table(w, f64);
 }
@@ -1150,11 +1145,7 @@ const void* Solver::twiddle_plain(int L, bool f64) {
     auto it = twiddles.find(key);
     if (it != twiddles.end()) return it->second;
     std::vector<double> w(2 * (size_t)L);
-    for (int q = 0; q < L; ++q) {
-        const long double a = -2.0L * (long double)M_PI * (long double)q / (long double)L;
-        w[2 * q] = (double)cosl(a);
-        w[2 * q + 1] = (double)sinl(a);
-    }
+    for (int q = 0; q < L; ++q) root_of_unity(q, L, &w[2 * q]);
     return twiddles[key] = upload_table(w, f64);
 }
 
